@@ -1895,27 +1895,27 @@ struct AdjointOps {
   static void jvp(const View<R> &V, const double *cvDotRef, double *rhsDotRef, double *work, cudaStream_t s) {
     const size_t nT = (size_t)V.nf + V.nb;
     AdjWork<R> W = carveAdjWork<R>(work, V.nc, nT);
-    kTanInit<R><<<blocks(V.nc), kBlock, 0, s>>>(V, W, cvDotRef);
-    if (V.p.spaceOrder > 1) kTanGrad<R><<<blocks(V.nc), kBlock, 0, s>>>(V, W);
-    if (isWeno(V.p)) kTanWeno<R><<<blocks(V.nc), kBlock, 0, s>>>(V, W);
-    kTanFlux<R><<<blocks((long long)nT), kBlock, 0, s>>>(V, W);
-    kTanGather<R><<<blocks(V.nc), kBlock, 0, s>>>(V, W, rhsDotRef);
+    kTanInit<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, cvDotRef);
+    if (V.p.spaceOrder > 1) kTanGrad<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
+    if (isWeno(V.p)) kTanWeno<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
+    kTanFlux<R><<<RFLU_GRID(V, (long long)nT, s)>>>(V, W);
+    kTanGather<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, rhsDotRef);
   }
   static void gradFwd(const View<R> &V, const AdjWork<R> &W, const double *lamRef, cudaStream_t s) {
-    if (V.p.reconst == 10) kAdjGradFwd<R, true><<<blocks(V.nc), kBlock, 0, s>>>(V, W, lamRef);
-    else kAdjGradFwd<R, false><<<blocks(V.nc), kBlock, 0, s>>>(V, W, lamRef);
+    if (V.p.reconst == 10) kAdjGradFwd<R, true><<<RFLU_GRID(V, V.nc, s)>>>(V, W, lamRef);
+    else kAdjGradFwd<R, false><<<RFLU_GRID(V, V.nc, s)>>>(V, W, lamRef);
     if (isWeno(V.p)) {
       if constexpr (Layout<R>::packed)
-        kAdjWenoFwdLanes<R><<<blocks((long long)V.nc * adjLanes<R>()), kBlock, 0, s>>>(V, W);
+        kAdjWenoFwdLanes<R><<<RFLU_GRID(V, (long long)V.nc * adjLanes<R>(), s)>>>(V, W);
       else
-        kAdjWenoFwd<R><<<blocks(V.nc), kBlock, 0, s>>>(V, W);
+        kAdjWenoFwd<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
     }
   }
   static void cellAdjoint(const View<R> &V, AdjWork<R> &W, double *cvBarRef, cudaStream_t s) {
-    if (V.p.reconst == 10 && V.p.spaceOrder > 1) kAdjCell1<R, true><<<blocks(V.nc), kBlock, 0, s>>>(V, W);
-    else kAdjCell1<R, false><<<blocks(V.nc), kBlock, 0, s>>>(V, W);
-    if (isWeno(V.p)) kAdjWeno<R><<<blocks((long long)V.nc * adjLanes<R>()), kBlock, 0, s>>>(V, W);
-    kAdjCell2<R><<<blocks(V.nc), kBlock, 0, s>>>(V, W, cvBarRef);
+    if (V.p.reconst == 10 && V.p.spaceOrder > 1) kAdjCell1<R, true><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
+    else kAdjCell1<R, false><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
+    if (isWeno(V.p)) kAdjWeno<R><<<RFLU_GRID(V, (long long)V.nc * adjLanes<R>(), s)>>>(V, W);
+    kAdjCell2<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, cvBarRef);
   }
   // The boundary faces' kernel (dual numbers through the patch fluxes; few
   // faces, a small grid) runs on a second stream beside the interior faces'
@@ -1926,17 +1926,17 @@ struct AdjointOps {
     const int nT = V.nf + V.nb;
     const bool roe2 = V.p.spaceOrder > 1 && V.p.spaceDiscr == 1;
     if (V.nf == 0 || V.nb == 0) {
-      if (nT > 0 && !(roe2 && V.nb == 0)) kAdjFace<R, false><<<blocks((long long)nT), kBlock, 0, s>>>(V, W, 0, nT);
-      else if (nT > 0) kAdjFace<R, true><<<blocks((long long)nT), kBlock, 0, s>>>(V, W, 0, nT);
+      if (nT > 0 && !(roe2 && V.nb == 0)) kAdjFace<R, false><<<RFLU_GRID(V, (long long)nT, s)>>>(V, W, 0, nT);
+      else if (nT > 0) kAdjFace<R, true><<<RFLU_GRID(V, (long long)nT, s)>>>(V, W, 0, nT);
       return;
     }
     SideStream &ss = sideStream();
     cudaEventRecord(ss.fork, s);
     cudaStreamWaitEvent(ss.stream, ss.fork, 0);
-    kAdjFace<R, false><<<blocks((long long)V.nb), kBlock, 0, ss.stream>>>(V, W, V.nf, nT);
+    kAdjFace<R, false><<<RFLU_GRID(V, (long long)V.nb, ss.stream)>>>(V, W, V.nf, nT);
     cudaEventRecord(ss.join, ss.stream);
-    if (roe2) kAdjFace<R, true><<<blocks((long long)V.nf), kBlock, 0, s>>>(V, W, 0, V.nf);
-    else kAdjFace<R, false><<<blocks((long long)V.nf), kBlock, 0, s>>>(V, W, 0, V.nf);
+    if (roe2) kAdjFace<R, true><<<RFLU_GRID(V, (long long)V.nf, s)>>>(V, W, 0, V.nf);
+    else kAdjFace<R, false><<<RFLU_GRID(V, (long long)V.nf, s)>>>(V, W, 0, V.nf);
     cudaStreamWaitEvent(s, ss.join, 0);
   }
   static void vjp(const View<R> &V, const double *rhsBarRef, double *cvBarRef, double *work, cudaStream_t s) {
@@ -1945,7 +1945,7 @@ struct AdjointOps {
     // every face-adjoint entry the cell kernels read is written by the face
     // kernels: no clearing of faceAdj here
     if (V.p.spaceOrder > 1) gradFwd(V, W, rhsBarRef, s);
-    else kAdjLambda<R><<<blocks(V.nc), kBlock, 0, s>>>(V, W, rhsBarRef);
+    else kAdjLambda<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, rhsBarRef);
     (void)nT;
     faceAdjoint(V, W, s);
     cellAdjoint(V, W, cvBarRef, s);
@@ -1954,7 +1954,7 @@ struct AdjointOps {
     const size_t nT = (size_t)V.nf + V.nb;
     AdjWork<R> W = carveAdjWork<R>(work, V.nc, nT);
     gradFwd(V, W, nullptr, s);
-    kLimiterBranches<R><<<blocks(V.nc), kBlock, 0, s>>>(V, W, outRef);
+    kLimiterBranches<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, outRef);
   }
   static void patchPressure(const View<R> &V, int ip, double *J, double *cvBarRef, double *work, cudaStream_t s) {
     const size_t nT = (size_t)V.nf + V.nb;

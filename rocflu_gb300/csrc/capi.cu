@@ -1379,6 +1379,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
 
   // ---- device upload -----------------------------------------------------------
   V.nc = nc; V.nf = nf; V.nb = nb;
+  RFLU_CUDA(cudaDeviceGetAttribute(&V.sms, cudaDevAttrMultiProcessorCount, device));
   int rc = 0;
 #define PUT(dst, src, T) if ((rc = put<T>(&(dst), src))) return rc
   if (mixed) {

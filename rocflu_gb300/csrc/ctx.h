@@ -91,6 +91,7 @@ template <> struct Layout<float> {
 template <typename R>
 struct View {
   int nc, nf, nb;             // cells, interior faces, boundary faces
+  int sms;                    // SMs of the device (launch shapes)
   // interior faces (storage order), renumbered cells; FP64 modes
   const int *fc1, *fc2;
   const R *fnx, *fny, *fnz, *fnm;   // unit normal and area

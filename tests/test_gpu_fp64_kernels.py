@@ -1,0 +1,33 @@
+"""FP64 kernels on the device at the sizes where a launch or a kernel branch
+changes, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from oracle.oracle import Oracle
+from rocflu_gb300 import cases, gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def _wavy(case, seed=5, amp=0.05):
+    """The case's state with every variable disturbed."""
+    rng = np.random.default_rng(seed)
+    cv = case.cv0 * (1.0 + amp * rng.standard_normal(case.cv0.shape))
+    cv[:, 1:4] += amp * rng.standard_normal((len(cv), 3))
+    return cv
+
+
+@pytest.mark.parametrize("nx", [1, 31, 33, 3041, 4871, 9728, 9729, 19457, 38913])
+def test_launch_shapes_bit_exact(gpu_lib, nx):
+    """Blocks of 32 to 256 threads and their remainders (4 nx cells): two
+    first-order steps, FP64_EXACT, equal to the oracle's bits."""
+    c = cases.sod(nx, 2, 2)
+    c.cv0 = _wavy(c)
+    c.num.dt_imposed = 1e-6
+    o = Oracle(c)
+    o.set_state(c.cv0)
+    n_o, t_o = o.run(2, 1.0)
+    r = gpu.Region(c, "fp64_exact")
+    n_g, t_g, rc = r.step(2, 1.0)
+    assert rc == 0 and n_g == n_o and t_g == t_o
+    np.testing.assert_array_equal(r.download()[0], o.state()[0])
