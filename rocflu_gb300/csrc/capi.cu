@@ -807,6 +807,7 @@ struct Ctx : CtxBase {
     W.prim = (R *)p;               p += bPrim;
     W.grad = (R *)p;               p += bGrad;
     if (V.gradRaw) { W.gradRaw = (R *)p; p += bRaw; }
+    W.wenoW = nullptr;  // the smoothing forms its weights itself: the scratch takes the same meshes
     W.flux = (R *)p;               p += bFlux;
     W.rhs = (R *)p;
     kPermuteIn<<<nblk(W.nc), 256, 0, stream>>>(cvDev, W.cv, W.refId, W.nc);
@@ -1518,6 +1519,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   if ((num->reconst == 1 || num->reconst == 2) && num->spaceOrder > 1 &&
       (rc = alloc(&V.gradRaw, Layout<R>::grad * (size_t)nc)))
     return rc;
+  if (!mixed && num->reconst == 2 && num->spaceOrder > 1 && (rc = alloc(&V.wenoW, 15 * (size_t)nc))) return rc;
   if ((rc = alloc(&V.rhsSum, 5 * (size_t)nc))) return rc;
   if ((rc = alloc(&V.flux, 5 * ((size_t)nf + nb)))) return rc;
   if ((rc = alloc(&V.rhs, 5 * (size_t)nc))) return rc;

@@ -153,6 +153,9 @@ struct View {
   // WENO smoothing (RECONST 1, 2): the unsmoothed gradients the gradient
   // kernels write, in the layout of grad, read by kWenoSmooth
   R *gradRaw;
+  // FP64 layouts, RECONST 2: each unsmoothed component's WENO weight (15 Nc);
+  // null: the smoothing forms them
+  R *wenoW;
   // mixed mode, adjoint of the LSQ gradient: the transposed stencil entry-
   // major (entry k of cell j at k*nc + j): d/|d|^2 with d = x_j - x_i for
   // the cell i whose stencil holds j, and i as int bits (-1 past the end)

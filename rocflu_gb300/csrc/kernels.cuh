@@ -526,6 +526,15 @@ __device__ inline void reflectGrad(const Qt *Q, S *g) {
     }
 }
 
+// FP64 layouts, WENO-XYZ: component k of cell i's unsmoothed gradient t enters
+// the averages of the cell and of every cell whose stencil holds it with the
+// weight w = 1/(t^2 + 1e-15) (RFLU_WENOGradCellsXYZFast_3D), formed once per
+// cell instead of once per (cell, member) pair.
+template <typename R>
+__device__ inline void storeWenoWeight(const View<R> &V, int k, int i, R t) {
+  V.wenoW[(size_t)k * V.nc + i] = R(1) / (t * t + R(1.0e-15));
+}
+
 // Gradient + limiter of one cell.
 // LSQ gradient: RFLU_ComputeGradCellsFast_3D (modflu/RFLU_ModDifferentiationCells.F90:
 // 931-1178) with the per-member weights precomputed at set-up.
@@ -1245,8 +1254,55 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<R>::v) kGradLimit(View<R> V)
     gradLimitPacked<false, false, -1>(V, i, g, dc + threadIdx.x, nullptr, 0);
   } else {
     gradLimitCell(V, PlainLoad<R>{V}, i, g);
+    if (V.wenoW) {
+#pragma unroll
+      for (int k = 0; k < 15; ++k) storeWenoWeight(V, k, i, g[k]);
+    }
   }
   storeGrad(V, i, g);
+}
+
+// The unlimited gradient (RECONST 0, 1, 2) of the FP64 layouts, one thread per
+// cell and variable (blockIdx.y): the same differences and sums as
+// gradLimitCell, five times the threads.  The arithmetic is the FP64 pipe's
+// either way; a small mesh gains the shorter chain per thread (four FP64
+// instructions per member instead of twenty, at 64 cycles each on a
+// sub-partition with one warp).  Measured with the smoothing pass below
+// (kWenoVar).
+template <typename R>
+__global__ void __launch_bounds__(kBlock) kGradVar(View<R> V) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= V.nc) return;
+  const int v = blockIdx.y;
+  const size_t n = V.nc;
+  const R *q = V.prim + v * n;
+  const R qi = q[i];
+  R gx = R(0), gy = R(0), gz = R(0);
+  const int se = V.stOff[i + 1];
+#pragma unroll 2
+  for (int s = V.stOff[i]; s < se; ++s) {
+    const int j = V.stIdx[s];
+    R qj = q[j];
+    if (V.stXf && v >= 1 && v <= 3) {  // a member seen reflected across symmetry patches
+      const int x = V.stXf[s];
+      if (x >= 0) {
+        const R u[3] = {V.prim[n + j], V.prim[2 * n + j], V.prim[3 * n + j]};
+        R y[3];
+        reflect3(V.xfQ + 9 * x, u, y);
+        qj = v == 1 ? y[0] : v == 2 ? y[1] : y[2];
+      }
+    }
+    const R d = qj - qi;
+    gx = gx + V.wx[s] * d;
+    gy = gy + V.wy[s] * d;
+    gz = gz + V.wz[s] * d;
+  }
+  const R g[3] = {gx, gy, gz};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    V.grad[(3 * v + c) * n + i] = g[c];
+    if (V.wenoW) storeWenoWeight(V, 3 * v + c, i, g[c]);
+  }
 }
 
 // Block minimum of a per-thread dt (warp shuffles, then one warp over the
@@ -1714,6 +1770,78 @@ __global__ void __launch_bounds__(kBlock) kWenoSmooth(View<R> V, const R *raw) {
                    },
                    g);
   storeGrad(V, i, g);
+}
+
+// WENO-XYZ of the FP64 layouts from the stored weights (storeWenoWeight), one
+// thread per cell and variable (blockIdx.y), with the simple limiter of
+// density and pressure.  An addition and a multiply-add per member and
+// component where kWenoSmooth recomputes each member's weight (a division and
+// one more); the sums run in the same order with the same operations, so the
+// results are the same bits.  A member seen reflected across symmetry patches
+// is another gradient: its weight is formed here.  Bound by the FP64 pipe.
+// Measured with kGradVar: 20 FP64_EXACT steps of 512 cells 13.1 -> 3.7 ms, 2
+// FP64 steps of a periodic 40^3 box 3.73 -> 2.56 ms.
+template <typename R>
+__global__ void __launch_bounds__(kBlock) kWenoVar(View<R> V, const R *raw) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= V.nc) return;
+  const int v = blockIdx.y;
+  const size_t n = V.nc, nb = V.nb;
+  const R *w = V.wenoW + 3 * v * n, *t = raw + 3 * v * n;
+  R sum[3], g[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    sum[c] = w[c * n + i];
+    g[c] = sum[c] * t[c * n + i];
+  }
+  const int se = V.stOff[i + 1];
+#pragma unroll 2
+  for (int s = V.stOff[i]; s < se; ++s) {
+    const int j = V.stIdx[s];
+    const int x = V.stXf ? V.stXf[s] : -1;
+    if (x >= 0) {
+      R tr[15];
+#pragma unroll
+      for (int k = 0; k < 15; ++k) tr[k] = raw[k * n + j];
+      reflectGrad(V.xfQ + 9 * x, tr);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const R tc = v == 0 ? tr[c] : v == 1 ? tr[3 + c] : v == 2 ? tr[6 + c] : v == 3 ? tr[9 + c] : tr[12 + c];
+        const R ww = R(1) / (tc * tc + R(1.0e-15));
+        sum[c] = sum[c] + ww;
+        g[c] = g[c] + ww * tc;
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const R ww = w[c * n + j];
+        sum[c] = sum[c] + ww;
+        g[c] = g[c] + ww * t[c * n + j];
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) g[c] = g[c] / sum[c];
+  if (v == 0 || v == 4) {
+    const R q = V.prim[v * n + i];
+    bool zero = false;
+    for (int e = V.cfOff[i]; e < V.cfOff[i + 1]; ++e) {
+      const int code = V.cfEnt[e];
+      R d[3];
+      if (code >= 0) {
+        faceOffset(V, code >> 1, code & 1, d);
+      } else {
+        const int b = -code - 1;
+        d[0] = V.bd[b];
+        d[1] = V.bd[nb + b];
+        d[2] = V.bd[2 * nb + b];
+      }
+      if (q + g[0] * d[0] + g[1] * d[1] + g[2] * d[2] <= R(0)) zero = true;
+    }
+    if (zero) g[0] = g[1] = g[2] = R(0);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) V.grad[(3 * v + c) * n + i] = g[c];
 }
 
 // Tiled WENO smoothing for the mixed mode: one tile of kTile Morton cells per
@@ -2529,10 +2657,30 @@ struct Launch {
     if (V.p.spaceOrder < 2) return;
     const View<R> W = rawView(V);
     if (V.tiled) launchTile<false>(W, s);
+    else if (unlimitedPerVar(V)) launchGradVar(W, s);
     else kGradLimit<R><<<RFLU_GRID(V, V.nc, s)>>>(W);
     if (weno(V)) smooth(V, s);
   }
+  // FP64 layouts: one thread per cell and variable (blockIdx.y).  The
+  // constrained gradients' rows run through a cell's variables in turn and
+  // keep the kernel with one thread per cell.
+  static bool unlimitedPerVar(const View<R> &V) {
+    return !Layout<R>::packed && (V.p.reconst == 0 || weno(V)) && !V.cSlot;
+  }
+  static void launchGradVar(const View<R> &V, cudaStream_t s) {
+    if constexpr (!Layout<R>::packed) {
+      const int b = shapeFor(V, 5LL * V.nc).block;
+      kGradVar<R><<<dim3((V.nc + b - 1) / b, 5), b, 0, s>>>(V);
+    }
+  }
   static void smooth(const View<R> &V, cudaStream_t s) {
+    if constexpr (!Layout<R>::packed) {
+      if (V.wenoW) {
+        const int b = shapeFor(V, 5LL * V.nc).block;
+        kWenoVar<R><<<dim3((V.nc + b - 1) / b, 5), b, 0, s>>>(V, V.gradRaw);
+        return;
+      }
+    }
     if (Layout<R>::packed && V.tiled)
       kWenoTile<R><<<(V.nc + kTile - 1) / kTile, kBlock, wenoTileSmemBytes(V), s>>>(V, V.gradRaw);
     else
