@@ -22,6 +22,7 @@
 #include "constr.h"
 #include "ctx.h"
 #include "errors.h"
+#include "fixedsum.h"
 #include "ops.h"
 #include "tiles.h"
 
@@ -318,6 +319,21 @@ struct Ctx : CtxBase {
     allocs.push_back(q);
     *p = (T *)q;
     return RFLU_OK;
+  }
+  // An array that only makes the context faster: null when the device is
+  // full, and the kernels that do without it run instead.
+  template <typename T>
+  bool allocOptional(T **p, size_t n) {
+    void *q = nullptr;
+    if (cudaMalloc(&q, n * sizeof(T)) != cudaSuccess) {
+      cudaGetLastError();
+      *p = nullptr;
+      return false;
+    }
+    bytesHeld += n * sizeof(T);
+    allocs.push_back(q);
+    *p = (T *)q;
+    return true;
   }
   template <typename T, typename S>
   int put(const T **dst, const std::vector<S> &src) {
@@ -1434,6 +1450,17 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
     }
   } else {
     PUT(V.wx, wx, R); PUT(V.wy, wy, R); PUT(V.wz, wz, R);
+    // the fixed-point sums' weights (configure fills them); the sums' scratch
+    // (seven values per cell) is the face-flux array
+    int w = 0;
+    for (int i = 0; i < nc; ++i) w = std::max(w, stOff[i + 1] - stOff[i]);
+    if (num->precision == RFLU_PREC_FP64 && num->spaceOrder > 1 && w > 0 && w <= kFixMaxTerms &&
+        5 * ((size_t)nf + nb) >= 7 * (size_t)nc) {
+      V.fxWidth = w;
+      if (!allocOptional(&V.fxW, 3 * (size_t)w * nc) || !allocOptional(&V.fxScale, nc) ||
+          !allocOptional(&V.fxIdx, (size_t)w * nc))
+        V.fxIdx = nullptr;
+    }
   }
   // transposed stencil (adjoint of the LSQ gradient, every mode)
   PUT(V.tsOff, tsOff, int); PUT(V.tsCell, tsCell, int); PUT(V.tsEnt, tsEnt, int);
@@ -1519,7 +1546,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   if ((num->reconst == 1 || num->reconst == 2) && num->spaceOrder > 1 &&
       (rc = alloc(&V.gradRaw, Layout<R>::grad * (size_t)nc)))
     return rc;
-  if (!mixed && num->reconst == 2 && num->spaceOrder > 1 && (rc = alloc(&V.wenoW, 15 * (size_t)nc))) return rc;
+  if (!mixed && num->reconst == 2 && num->spaceOrder > 1) allocOptional(&V.wenoW, 15 * (size_t)nc);
   if ((rc = alloc(&V.rhsSum, 5 * (size_t)nc))) return rc;
   if ((rc = alloc(&V.flux, 5 * ((size_t)nf + nb)))) return rc;
   if ((rc = alloc(&V.rhs, 5 * (size_t)nc))) return rc;

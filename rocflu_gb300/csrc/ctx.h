@@ -133,6 +133,14 @@ struct View {
   // C2C stencil CSR and per-member least-squares weights
   const int *stOff, *stIdx;
   const R *wx, *wy, *wz;
+  // RFLU_PREC_FP64: the stencil entry-major (entry k of cell i at k*nc + i)
+  // for the fixed-point sums (fixedsum.h): member (-1 past the end), the
+  // weights' halves (component c at (c*fxWidth + k)*nc + i) in units of
+  // 2^(fxScale - 55); null: the FP64 sums
+  int *fxIdx;
+  int2 *fxW;
+  int *fxScale;
+  int fxWidth;
   const double *vol;
   const R *epsq;                    // Venkatakrishnan eps^2 = (vol^(1/3))^3 per cell
   // mixed mode: the LSQ weights w_j = L d_j / |d_j|^2 of a cell share one

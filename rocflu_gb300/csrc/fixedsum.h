@@ -1,0 +1,139 @@
+// Sums of products of doubles on the integer pipe.
+//
+// The GB300 runs one FP64 instruction per sub-partition in about 64 cycles and
+// a 32x32+64-bit integer multiply-add in 2.3 (measured), so a sum of products
+// whose terms share a scale is formed in fixed point: every factor becomes a
+// 56-bit integer in units of its block's largest magnitude, is split into two
+// 28-bit halves, and the partial products are accumulated exactly in 64-bit
+// integers (Karatsuba: three multiplies per product).  The only rounding is
+// that of the factors to their units, 2^-55 of the block's largest magnitude,
+// and of the result to a double; a sum in FP64 rounds every term and every
+// partial sum at 2^-53 of their size.
+//
+// Host and device code (no CUDA types): tests/test_fixedsum_cpu.py compares it
+// with exact rational sums.
+#pragma once
+#include <cstdint>
+#include <cstring>
+
+#ifdef __CUDACC__
+#define RFLU_HD __host__ __device__
+#else
+#define RFLU_HD
+#endif
+
+namespace rflu {
+
+// A finite double as (signed mantissa << 2) * 2^(e - 1077), e its biased
+// exponent; e = 0 only for zero.  kFixBad marks what the fixed-point sums do
+// not take (denormals, infinities, NaN, magnitudes outside about 2^-500 ..
+// 2^500): it is larger than every other e, so that it survives a maximum.
+constexpr int kFixBad = 4095, kFixEmin = 523, kFixEmax = 1523;
+constexpr int kFixMaxTerms = 64;   // terms per sum that cannot overflow
+constexpr int kFixBadScale = 1 << 20;
+
+struct FixNum {
+  int64_t m;
+  int e;
+};
+RFLU_HD inline FixNum fixOf(double x) {
+  uint64_t b;
+#ifdef __CUDA_ARCH__
+  b = (uint64_t)__double_as_longlong(x);
+#else
+  std::memcpy(&b, &x, 8);
+#endif
+  FixNum r;
+  const int e = (int)((b >> 52) & 0x7ff);
+  const int64_t m = (int64_t)(((b & 0xfffffffffffffull) | 0x10000000000000ull) << 2);
+  const bool zero = (b << 1) == 0;
+  r.m = zero ? 0 : ((int64_t)b < 0 ? -m : m);
+  r.e = zero ? 0 : (e < kFixEmin || e > kFixEmax) ? kFixBad : e;
+  return r;
+}
+
+// The number in units of 2^(eMax - 1077), eMax >= e (rounded down).
+RFLU_HD inline int64_t fixAt(int64_t m, int e, int eMax) {
+  const int s = eMax - e;
+  return m >> (s < 63 ? s : 63);
+}
+
+// A weight in units of 2^(x - 55) with |w| < 2^x, in two signed halves: w =
+// (hi * 2^28 + lo) units, |hi| <= 2^27, -2^27 <= lo < 2^27.
+struct FixHalves {
+  int hi, lo;
+};
+RFLU_HD inline FixHalves fixSplit(int64_t v) {
+  FixHalves h;
+  h.hi = (int)((v + (1 << 27)) >> 28);
+  h.lo = (int)((uint32_t)v - ((uint32_t)h.hi << 28));
+  return h;
+}
+
+// One sum of products; the weights' halves and the differences' halves are
+// formed once per member and used in 15 sums.  |difference| <= 2^56 units.
+struct FixSum {
+  int64_t hh, ss, ll;
+};
+RFLU_HD inline void fixAdd(FixSum &a, int wh, int wl, int ws, int dh, int dl, int ds) {
+  a.hh += (int64_t)wh * dh;
+  a.ll += (int64_t)wl * dl;
+  a.ss += (int64_t)ws * ds;  // ws = wh + wl, ds = dh + dl: hh + ll + the cross terms
+}
+
+RFLU_HD inline int fixClz(uint64_t x) {
+#ifdef __CUDA_ARCH__
+  return __clzll((long long)x);
+#else
+  return __builtin_clzll(x);
+#endif
+}
+
+// The sum as a double: units of 2^scale; rounded to nearest.
+RFLU_HD inline double fixResult(const FixSum &a, int scale) {
+  const int64_t mid = a.ss - a.hh - a.ll;
+  // a.hh * 2^56 + mid * 2^28 + a.ll as h * 2^56 + low, 0 <= low < 2^56
+  const int64_t m1 = mid + (a.ll >> 28);
+  int64_t h = a.hh + (m1 >> 28);
+  uint64_t low = ((uint64_t)(m1 & 0xfffffff) << 28) | (uint64_t)(a.ll & 0xfffffff);
+  const bool neg = h < 0;
+  if (neg) {
+    h = low ? ~h : -h;
+    low = low ? (1ull << 56) - low : 0;
+  }
+  const uint64_t H = (uint64_t)h, L = low << 8;
+  if ((H | L) == 0) return 0.0;
+  int lz;
+  uint64_t top;
+  if (H) {
+    lz = fixClz(H);
+    top = (H << lz) | (lz ? L >> (64 - lz) : 0);
+  } else {
+    const int l = fixClz(L);
+    lz = 64 + l;
+    top = L << l;
+  }
+  // top's leading bit stands for 2^(119 - lz) units
+  const int e = 119 - lz + scale + 1022;
+  const uint64_t bits = ((uint64_t)e << 52) + (top >> 11) + ((top >> 10) & 1) + (neg ? 1ull << 63 : 0);
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)bits);
+#else
+  double d;
+  std::memcpy(&d, &bits, 8);
+  return d;
+#endif
+}
+
+// |w| < 2^x for the largest magnitude of a block of weights: its biased
+// exponent minus 1022; kFixBadScale for what fixOf does not take (or none).
+RFLU_HD inline int fixScale(int eMax) { return (eMax == 0 || eMax == kFixBad) ? kFixBadScale : eMax - 1022; }
+// A weight of that block in units of 2^(x - 55), rounded to nearest.
+RFLU_HD inline int64_t fixWeight(double w, int eMax) {
+  const FixNum f = fixOf(w);
+  const int s = eMax - f.e;
+  if (s > 60) return 0;
+  return s == 0 ? f.m : ((f.m >> (s - 1)) + 1) >> 1;
+}
+
+}  // namespace rflu

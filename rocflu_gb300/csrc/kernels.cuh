@@ -20,6 +20,7 @@
 #include "convert.cuh"
 #include "ctx.h"
 #include "dual.cuh"
+#include "fixedsum.h"
 #include "physics.cuh"
 
 namespace rflu {
@@ -545,6 +546,8 @@ __device__ inline void storeWenoWeight(const View<R> &V, int k, int i, R t) {
 // two face sweeps become two loops over the cell's own faces.
 // ---------------------------------------------------------------------------
 template <typename R, typename L>
+__device__ inline void limitCell(const View<R> &V, const L &ld, int i, const typename L::S *q, typename L::S *g);
+template <typename R, typename L>
 __device__ inline void gradLimitCell(const View<R> &V, const L &ld, int i, typename L::S *g) {
   using S = typename L::S;
   S q[5];
@@ -622,6 +625,13 @@ __device__ inline void gradLimitCell(const View<R> &V, const L &ld, int i, typen
       if (sl >= 0) constrainedGrad(V, ld, i, sl, q, g);
     }
   }
+  limitCell(V, ld, i, q, g);
+}
+
+// The limiter of gradLimitCell on the unlimited gradient g of cell i.
+template <typename R, typename L>
+__device__ inline void limitCell(const View<R> &V, const L &ld, int i, const typename L::S *q, typename L::S *g) {
+  using S = typename L::S;
   const int rc = V.p.reconst;
   const int cb = V.cfOff[i], ce = V.cfOff[i + 1];
   if (rc == 10 || rc == 100 || rc == 11) {
@@ -1305,6 +1315,280 @@ __global__ void __launch_bounds__(kBlock) kGradVar(View<R> V) {
   }
 }
 
+__device__ inline void cpAsync16(void *smemDst, const void *gSrc) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smemDst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gSrc) : "memory");
+}
+__device__ inline void cpAsync4(void *smemDst, const void *gSrc) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smemDst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gSrc) : "memory");
+}
+__device__ inline void cpAsyncCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ inline void cpAsyncWait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+__device__ inline void cpAsync8(void *smemDst, const void *gSrc) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smemDst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gSrc) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// The least-squares sums of RFLU_PREC_FP64 on the integer pipe (fixedsum.h).
+//
+// Per member the fit takes 15 multiply-adds and 5 differences: 20 FP64
+// instructions, 1,300 cycles of a sub-partition; as 45 integer multiply-adds
+// on 28-bit halves plus the conversions 290 instructions.  Bound by issue and
+// the latency of the members' gathers at 12 warps per SM (168 registers).
+// Measured, 421,875 hexahedra of 26 members, FP64 pipe 100% busy before: about
+// 440 us of the gradient kernel -> 235 us in the three kernels below; 131,712
+// tetrahedra of 40: 260 -> 132 us.  The block whose largest
+// magnitude sets the unit is the cell's own stencil, per variable, so the
+// rounding is 2^-55 of the largest value the fit sees, below that of the FP64
+// differences and partial sums.  Cells the fixed point does not take
+// (values beyond 2^+-500, denormals, infinities, NaN, reflected members, more
+// than kFixMaxTerms members) run the FP64 loop.  FP64_EXACT keeps the FP64
+// loop for its bits, the mixed mode its FP32 sums.
+// ---------------------------------------------------------------------------
+#ifdef RFLU_FIXED_SUMS
+constexpr bool kFixedSums = true;
+#else
+constexpr bool kFixedSums = false;
+#endif
+constexpr int kFixBlock = 128;
+constexpr int kFixDepth = 8;  // members in flight per thread (a power of two)
+
+// Five fields as the sums read them, structure-of-arrays over the cells:
+// signed mantissas (fixOf) at m[v*nc + i], the biased exponents in ten bits
+// each (kFixEmin taken as 1, zero as 0, what the sums do not take as
+// kFixExpBad) at e[i], and the largest exponents of cell i's stencil at
+// eMax[i].  A warp's gather of one 8-byte array touches the few 128-byte lines
+// its 32 neighbouring members share; as one 64-byte record per cell every
+// lane touched its own (421,875 hexahedra: exponents 43 -> 24 us, sums 218 ->
+// 203 us).  The largest exponents have a kernel of their own: a gather of 8 bytes per member hides
+// its latency behind many warps, which the kernel of the sums, with its 90
+// accumulator registers, does not have.
+constexpr int kFixExpBad = 1023;
+struct FixFields {
+  long long *m;
+  unsigned long long *e, *eMax;
+};
+inline FixFields fixFields(double *scratch, size_t nc) {
+  return {reinterpret_cast<long long *>(scratch), reinterpret_cast<unsigned long long *>(scratch + 5 * nc),
+          reinterpret_cast<unsigned long long *>(scratch + 6 * nc)};
+}
+__device__ inline unsigned fixExpOf(unsigned long long w, int v) { return (unsigned)(w >> (10 * v)) & 1023u; }
+
+template <typename R>
+__global__ void __launch_bounds__(kBlock) kFixRecords(const R *q, FixFields F, int nc) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nc) return;
+  unsigned long long w = 0;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const FixNum f = fixOf((double)q[(size_t)k * nc + i]);
+    F.m[(size_t)k * nc + i] = f.m;
+    const int e = f.e == 0 ? 0 : f.e == kFixBad ? kFixExpBad : f.e - kFixEmin + 1;
+    w |= (unsigned long long)e << (10 * k);
+  }
+  F.e[i] = w;
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kBlock) kFixExponents(View<R> V, FixFields F) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= V.nc) return;
+  const size_t n = V.nc;
+  const int cnt = V.stOff[i + 1] - V.stOff[i];
+  unsigned m[5];
+  const unsigned long long own = F.e[i];
+#pragma unroll
+  for (int v = 0; v < 5; ++v) m[v] = fixExpOf(own, v);
+#pragma unroll 4
+  for (int k = 0; k < cnt; ++k) {
+    const unsigned long long e = F.e[V.fxIdx[k * n + i]];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) m[v] = max(m[v], fixExpOf(e, v));
+  }
+  unsigned long long w = 0;
+#pragma unroll
+  for (int v = 0; v < 5; ++v) w |= (unsigned long long)m[v] << (10 * v);
+  F.eMax[i] = w;
+}
+
+// The members and weights of View::fxIdx / fxW / fxScale from the stencil CSR
+// (once per context).
+template <typename R>
+__global__ void __launch_bounds__(kBlock) kFixWeights(View<R> V) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= V.nc) return;
+  const size_t n = V.nc;
+  const int sb = V.stOff[i], cnt = V.stOff[i + 1] - sb;
+  int eMax = 0;
+  bool ok = cnt <= kFixMaxTerms;
+  for (int s = sb; s < sb + cnt; ++s) {
+    eMax = max(eMax, max(fixOf((double)V.wx[s]).e, max(fixOf((double)V.wy[s]).e, fixOf((double)V.wz[s]).e)));
+    if (V.stXf && V.stXf[s] >= 0) ok = false;
+  }
+  const int scale = fixScale(eMax);
+  V.fxScale[i] = ok ? scale : kFixBadScale;
+  for (int k = 0; k < V.fxWidth; ++k) {
+    const bool on = k < cnt;
+    V.fxIdx[k * n + i] = on ? V.stIdx[sb + k] : -1;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      FixHalves h{0, 0};
+      if (on && ok && scale != kFixBadScale)
+        h = fixSplit(fixWeight((double)(c == 0 ? V.wx : c == 1 ? V.wy : V.wz)[sb + k], eMax));
+      V.fxW[(c * (size_t)V.fxWidth + k) * n + i] = make_int2(h.hi, h.lo);
+    }
+  }
+}
+
+// The unlimited gradients of the five fields q (SoA) into out (SoA, 15
+// components); F holds q's mantissas and exponents.  primal: q is the view's
+// primitive state, whose constrained cells are fitted with their constraint
+// rows and whose WENO weights are stored.  Members and weights are entry-major,
+// so a warp's loads of them are contiguous.
+template <typename R>
+__global__ void __launch_bounds__(kFixBlock, 3) kGradFixed(View<R> V, const R *q, FixFields F, R *out, bool primal) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= V.nc) return;
+  const size_t n = V.nc;
+  const int cnt = V.stOff[i + 1] - V.stOff[i];
+  const unsigned long long ew = F.eMax[i];  // the stencil's largest exponents
+  unsigned emax[5];
+#pragma unroll
+  for (int v = 0; v < 5; ++v) emax[v] = fixExpOf(ew, v);
+  const int scale = V.fxScale[i];
+  R g[15];
+  if (scale != kFixBadScale && max(max(max(emax[0], emax[1]), max(emax[2], emax[3])), emax[4]) != kFixExpBad) {
+    // a cell's five values in units of the stencil's exponents: the ten-bit
+    // differences of all five come from one subtraction (no field borrows)
+    auto load = [&](int j, long long *m, unsigned long long &e) {
+#pragma unroll
+      for (int v = 0; v < 5; ++v) m[v] = F.m[v * n + j];
+      e = F.e[j];
+    };
+    auto atScale = [&](long long *m, unsigned long long e) {
+      const unsigned long long d = ew - e;
+#pragma unroll
+      for (int v = 0; v < 5; ++v) m[v] = m[v] >> min(fixExpOf(d, v), 63u);
+    };
+    long long own[5];
+    unsigned long long eo;
+    load(i, own, eo);
+    atScale(own, eo);
+    FixSum a[15];
+#pragma unroll
+    for (int k = 0; k < 15; ++k) a[k] = FixSum{0, 0, 0};
+    // Members and weights stream from HBM once: each thread copies its own
+    // into a ring in shared memory kFixDepth members ahead (no other thread
+    // reads them, so no barrier), and loads member k + 1's record while it sums
+    // member k.
+    __shared__ int2 ringW[kFixDepth][3][kFixBlock];
+    __shared__ int ringJ[kFixDepth][kFixBlock];
+    const int t = threadIdx.x;
+    const size_t wStride = (size_t)V.fxWidth * n;
+    auto fetch = [&](int k) {
+      if (k < cnt) {
+        const int slot = k % kFixDepth;
+        const size_t at = (size_t)k * n + i;
+        cpAsync4(&ringJ[slot][t], V.fxIdx + at);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) cpAsync8(&ringW[slot][c][t], V.fxW + c * wStride + at);
+      }
+      cpAsyncCommit();
+    };
+#pragma unroll
+    for (int k = 0; k < kFixDepth; ++k) fetch(k);
+    long long x[5];
+    unsigned long long ex = 0;
+    cpAsyncWait<kFixDepth - 1>();
+    if (cnt > 0) load(ringJ[0][t], x, ex);
+    for (int k = 0; k < cnt; ++k) {
+      cpAsyncWait<kFixDepth - 2>();  // member k + 1 has landed
+      const int slot = k % kFixDepth;
+      long long xn[5];
+      unsigned long long en;
+      load(k + 1 < cnt ? ringJ[(k + 1) % kFixDepth][t] : i, xn, en);
+      atScale(x, ex);
+      int2 w[3];
+      int ws[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        w[c] = ringW[slot][c][t];
+        ws[c] = w[c].x + w[c].y;
+      }
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        const FixHalves d = fixSplit(x[v] - own[v]);
+        const int ds = d.hi + d.lo;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) fixAdd(a[3 * v + c], w[c].x, w[c].y, ws[c], d.hi, d.lo, ds);
+      }
+#pragma unroll
+      for (int v = 0; v < 5; ++v) x[v] = xn[v];
+      ex = en;
+      fetch(k + kFixDepth);  // into the slot just read
+    }
+#pragma unroll
+    for (int k = 0; k < 15; ++k) g[k] = (R)fixResult(a[k], scale - 55 + (int)emax[k / 3] + kFixEmin - 1 - 1077);
+  } else {
+    R qi[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) qi[v] = q[v * n + i];
+#pragma unroll
+    for (int k = 0; k < 15; ++k) g[k] = R(0);
+    for (int s = V.stOff[i]; s < V.stOff[i + 1]; ++s) {
+      const int j = V.stIdx[s];
+      R qj[5];
+#pragma unroll
+      for (int v = 0; v < 5; ++v) qj[v] = q[v * n + j];
+      if (V.stXf && V.stXf[s] >= 0) {
+        const R u[3] = {qj[1], qj[2], qj[3]};
+        reflect3(V.xfQ + 9 * V.stXf[s], u, qj + 1);
+      }
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        const R d = qj[v] - qi[v];
+        g[3 * v] = g[3 * v] + V.wx[s] * d;
+        g[3 * v + 1] = g[3 * v + 1] + V.wy[s] * d;
+        g[3 * v + 2] = g[3 * v + 2] + V.wz[s] * d;
+      }
+    }
+  }
+  if (primal && V.cSlot) {
+    const int sl = V.cSlot[i];
+    if (sl >= 0) {
+      R qi[5];
+#pragma unroll
+      for (int v = 0; v < 5; ++v) qi[v] = q[v * n + i];
+      constrainedGrad(V, PlainLoad<R>{V}, i, sl, qi, g);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 15; ++k) {
+    out[k * n + i] = g[k];
+    if (primal && V.wenoW) storeWenoWeight(V, k, i, g[k]);
+  }
+}
+
+// The limiter alone, on the unlimited gradients in V.grad (FP64 layouts).
+template <typename R>
+__global__ void __launch_bounds__(kBlock) kLimit(View<R> V) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= V.nc) return;
+  const size_t n = V.nc;
+  const PlainLoad<R> ld{V};
+  R q[5], g[15];
+  ld.prim5(i, q);
+#pragma unroll
+  for (int k = 0; k < 15; ++k) g[k] = V.grad[k * n + i];
+  limitCell(V, ld, i, q, g);
+  storeGrad(V, i, g);
+}
+
 // Block minimum of a per-thread dt (warp shuffles, then one warp over the
 // warp minima) folded into one atomicMin on the bit pattern of the positive
 // double (IEEE order of positive doubles = order of their bit patterns).
@@ -1332,20 +1616,6 @@ __device__ inline void blockMinDt(Scalars *sc, double dt) {
 // variant with the time-step sum holds more per-cell state and runs at two
 // (up to 128 registers) instead of spilling at three.
 static_assert(kTile == kBlock, "one thread per cell of a tile");
-
-__device__ inline void cpAsync16(void *smemDst, const void *gSrc) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smemDst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gSrc) : "memory");
-}
-__device__ inline void cpAsync4(void *smemDst, const void *gSrc) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smemDst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gSrc) : "memory");
-}
-__device__ inline void cpAsyncCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ inline void cpAsyncWait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
 
 // One tile buffer: 8 floats per staged record, then the tile's stencil ids
 // as whole 16-byte words of stLoc (maxTileSt ids plus the misalignment of
@@ -1778,7 +2048,8 @@ __global__ void __launch_bounds__(kBlock) kWenoSmooth(View<R> V, const R *raw) {
 // component where kWenoSmooth recomputes each member's weight (a division and
 // one more); the sums run in the same order with the same operations, so the
 // results are the same bits.  A member seen reflected across symmetry patches
-// is another gradient: its weight is formed here.  Bound by the FP64 pipe.
+// is another gradient: its weight is formed here, as are all of them where the
+// view holds none (rflu_gpu_residual_static).  Bound by the FP64 pipe.
 // Measured with kGradVar: 20 FP64_EXACT steps of 512 cells 13.1 -> 3.7 ms, 2
 // FP64 steps of a periodic 40^3 box 3.73 -> 2.56 ms.
 template <typename R>
@@ -1787,12 +2058,14 @@ __global__ void __launch_bounds__(kBlock) kWenoVar(View<R> V, const R *raw) {
   if (i >= V.nc) return;
   const int v = blockIdx.y;
   const size_t n = V.nc, nb = V.nb;
-  const R *w = V.wenoW + 3 * v * n, *t = raw + 3 * v * n;
+  const R *w = V.wenoW ? V.wenoW + 3 * v * n : nullptr, *t = raw + 3 * v * n;
+  auto weight = [](R tc) { return R(1) / (tc * tc + R(1.0e-15)); };
   R sum[3], g[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    sum[c] = w[c * n + i];
-    g[c] = sum[c] * t[c * n + i];
+    const R tc = t[c * n + i];
+    sum[c] = w ? w[c * n + i] : weight(tc);
+    g[c] = __dmul_rn(sum[c], tc);  // rounded by itself, whatever the loop below is compiled to
   }
   const int se = V.stOff[i + 1];
 #pragma unroll 2
@@ -1807,16 +2080,17 @@ __global__ void __launch_bounds__(kBlock) kWenoVar(View<R> V, const R *raw) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const R tc = v == 0 ? tr[c] : v == 1 ? tr[3 + c] : v == 2 ? tr[6 + c] : v == 3 ? tr[9 + c] : tr[12 + c];
-        const R ww = R(1) / (tc * tc + R(1.0e-15));
+        const R ww = weight(tc);
         sum[c] = sum[c] + ww;
         g[c] = g[c] + ww * tc;
       }
     } else {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const R ww = w[c * n + j];
+        const R tc = t[c * n + j];
+        const R ww = w ? w[c * n + j] : weight(tc);
         sum[c] = sum[c] + ww;
-        g[c] = g[c] + ww * t[c * n + j];
+        g[c] = g[c] + ww * tc;
       }
     }
   }
@@ -2660,9 +2934,28 @@ struct Launch {
     if (V.p.spaceOrder < 2) return;
     const View<R> W = rawView(V);
     if (V.tiled) launchTile<false>(W, s);
-    else if (unlimitedPerVar(V)) launchGradVar(W, s);
+    else if (fixedSums(V)) {
+      launchFixed(W, W.prim, W.grad, true, s);
+      if (V.p.reconst == 10 || V.p.reconst == 100 || V.p.reconst == 11) launchLimit(W, s);
+    } else if (unlimitedPerVar(V)) launchGradVar(W, s);
     else kGradLimit<R><<<RFLU_GRID(V, V.nc, s)>>>(W);
     if (weno(V)) smooth(V, s);
+  }
+  // RFLU_PREC_FP64 with its fixed-point weights: the sums of five fields on
+  // the integer pipe.  Their records take the face-flux array, which holds
+  // nothing between a stage's update and its fluxes.
+  static bool fixedSums(const View<R> &V) { return kFixedSums && !Layout<R>::packed && V.fxIdx; }
+  static void launchFixed(const View<R> &V, const R *q, R *out, bool primal, cudaStream_t s) {
+    if constexpr (kFixedSums && !Layout<R>::packed) {
+      const FixFields F = fixFields(V.flux, V.nc);
+      kFixRecords<R><<<RFLU_GRID(V, V.nc, s)>>>(q, F, V.nc);
+      kFixExponents<R><<<RFLU_GRID(V, V.nc, s)>>>(V, F);
+      const int b = std::min(kFixBlock, shapeFor(V, V.nc).block);
+      kGradFixed<R><<<(V.nc + b - 1) / b, b, 0, s>>>(V, q, F, out, primal);
+    }
+  }
+  static void launchLimit(const View<R> &V, cudaStream_t s) {
+    if constexpr (kFixedSums && !Layout<R>::packed) kLimit<R><<<RFLU_GRID(V, V.nc, s)>>>(V);
   }
   // FP64 layouts: one thread per cell and variable (blockIdx.y).  The
   // constrained gradients' rows run through a cell's variables in turn and
@@ -2678,7 +2971,7 @@ struct Launch {
   }
   static void smooth(const View<R> &V, cudaStream_t s) {
     if constexpr (!Layout<R>::packed) {
-      if (V.wenoW) {
+      if (V.p.reconst == 2) {
         const int b = shapeFor(V, 5LL * V.nc).block;
         kWenoVar<R><<<dim3((V.nc + b - 1) / b, 5), b, 0, s>>>(V, V.gradRaw);
         return;
@@ -2733,6 +3026,9 @@ struct Launch {
     if (V.tsW) kTsWeights<R><<<RFLU_GRID(V, V.nc, s)>>>(V);
   }
   static void configure(const View<R> &V) {
+    if constexpr (kFixedSums && !Layout<R>::packed) {
+      if (V.fxIdx) kFixWeights<R><<<RFLU_GRID(V, V.nc, 0)>>>(V);
+    }
     if (V.tiled) {
       setTileSmem<false, 0>(V); setTileSmem<false, 10>(V); setTileSmem<false, 100>(V); setTileSmem<false, 11>(V);
       setTileSmem<true, 0>(V); setTileSmem<true, 10>(V); setTileSmem<true, 100>(V); setTileSmem<true, 11>(V);

@@ -1,5 +1,6 @@
 // Kernel instantiation of the fp64 mode: FP64, fused multiply-add allowed (-fmad=true).
 #define RFLU_NS fp64
+#define RFLU_FIXED_SUMS
 #include "kernels.cuh"
 #include "adjoint.cuh"
 #include "ops.h"

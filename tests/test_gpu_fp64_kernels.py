@@ -53,3 +53,51 @@ def test_gradients_by_variable_bit_exact(gpu_lib, mesh, reconst):
     rhs_g, grad_g = gpu.Region(c, "fp64_exact").residual(c.cv0)
     np.testing.assert_array_equal(grad_g, grad_o)
     np.testing.assert_array_equal(rhs_g, rhs_o)
+
+
+@pytest.mark.parametrize("mesh", ["hex", "tets", "periodic", "symmetry", "constrained"])
+@pytest.mark.parametrize("state", ["wavy", "wide", "extreme", "still"])
+def test_fixed_point_gradients(gpu_lib, mesh, state):
+    """The least-squares sums of the fp64 mode in fixed point against the
+    FP64_EXACT ones (unlimited gradients): values near each other, values
+    spread over ten orders of magnitude, magnitudes outside the fixed point's
+    range (the FP64 loop), a uniform state.  Bound: 1e-14 of the largest
+    weight sum times the largest difference, per cell and variable."""
+    num = cases.Numerics(space_order=2, space_discr=cases.DISCR_HLLC, reconst=cases.RECONST_NONE, cfl=0.4)
+    if mesh == "tets":
+        c = cases.adjoint_tets(4, num=num)
+    elif mesh == "symmetry":
+        c = cases.mirror_box(5, axes=(0, 1, 2), num=num)
+    elif mesh == "periodic":
+        c = cases.gas_jump_periodic(5)
+        c.num.reconst = cases.RECONST_NONE
+    else:
+        c = cases.shock_sphere(7, num=num)
+    if mesh == "constrained":
+        c.num.c_reconst = 1
+    rng = np.random.default_rng(9)
+    n = len(c.cv0)
+    rho, p = 1.0 + 0.3 * rng.random(n), 1.0 + 0.3 * rng.random(n)
+    u = rng.standard_normal((n, 3))
+    if state == "wide":
+        rho, p = 10.0 ** rng.uniform(-5, 5, n), 10.0 ** rng.uniform(-5, 5, n)
+        u = u * 10.0 ** rng.uniform(-8, 0, (n, 3))
+    elif state == "extreme":
+        u[::3, 0] *= 1e-160
+        u[1::3, 1] = 1e-310
+        u[:, 2] = 0.0
+    elif state == "still":
+        rho, p, u = np.ones(n), np.ones(n), np.zeros((n, 3))
+    c.cv0 = cases.conserved(rho, u[:, 0], u[:, 1], u[:, 2], p, c.num.gamma)
+    _, g = gpu.Region(c, "fp64").residual(c.cv0)
+    _, ref = gpu.Region(c, "fp64_exact").residual(c.cv0)
+    if state == "still":
+        np.testing.assert_array_equal(g, 0.0)
+        return
+    # per variable the largest value over the smallest spacing of the mesh
+    # bounds a cell's weights times differences; 40 members, FP64 rounding
+    grid = gpu.Setup(c)
+    h = grid.vol.min() ** (1 / 3)
+    prim = np.stack([rho, u[:, 0], u[:, 1], u[:, 2], p], axis=1)
+    scale = np.abs(prim).max(axis=0) / h
+    assert (np.abs(g - ref).max(axis=2) / np.maximum(scale, 1e-300)).max() < 1e-14
