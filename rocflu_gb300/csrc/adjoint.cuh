@@ -175,11 +175,11 @@ __device__ inline void primFromCv(const Params &P, const S *cv, S *q, S *dv) {
   const S gc = S(8314.3 / P.gvMol);
   const S g = S(P.gvCp / (P.gvCp - 8314.3 / P.gvMol));
   S r = cv[0];
-  S ir = S(1) / r;
+  S ir = div_(S(1), r);
   S Eo = ir * cv[4];
   S Vm2 = ir * ir * (cv[1] * cv[1] + cv[2] * cv[2] + cv[3] * cv[3]);
   S p = (g - S(1)) * r * (Eo - S(0.5) * Vm2);
-  S t = p / (r * gc);
+  S t = div_(p, r * gc);
   dv[0] = p;
   dv[1] = t;
   dv[2] = sqrt_(g * gc * t);
@@ -394,7 +394,7 @@ template <typename S>
 __device__ inline S venkat(S dext, S d2, S epsq) {
   S numer = (dext * dext + epsq) * d2 + S(2) * d2 * d2 * dext;
   S denom = d2 * (dext * dext + S(2) * d2 * d2 + dext * d2 + epsq);
-  return numer / (denom + S(1.0e-12));
+  return div_(numer, denom + S(1.0e-12));
 }
 
 // The eigen-frame velocity limiter of one cell (RECONST 10,
@@ -471,8 +471,8 @@ __device__ inline void velFrameForward(const View<R> &V, const L &ld, int i, con
       pr = pr + A[3 * j + 1] * du[1];
       pr = pr + A[3 * j + 2] * du[2];
       if (code >= 0 && (code & 1)) pr = -pr;
-      if (pr < dmn[j]) { dmn[j] = pr; nmn[j] = other; }
-      if (pr > dmx[j]) { dmx[j] = pr; nmx[j] = other; }
+      if (less_(pr, dmn[j])) { dmn[j] = pr; nmn[j] = other; }
+      if (less_(dmx[j], pr)) { dmx[j] = pr; nmx[j] = other; }
     }
   }
 #pragma unroll
@@ -499,12 +499,12 @@ __device__ inline void velFrameForward(const View<R> &V, const L &ld, int i, con
       pr = pr + A[3 * j] * sh[0];
       pr = pr + A[3 * j + 1] * sh[1];
       pr = pr + A[3 * j + 2] * sh[2];
-      if (pr > R(0)) {
-        const R t = dmx[j] / pr;
-        if (t < F.alRaw[j]) { F.alRaw[j] = t; F.side[j] = 1; F.face[j] = e; F.nb[j] = nmx[j]; F.dext[j] = dmx[j]; F.pext[j] = pr; }
-      } else if (pr < R(0)) {
-        const R t = dmn[j] / pr;
-        if (t < F.alRaw[j]) { F.alRaw[j] = t; F.side[j] = 2; F.face[j] = e; F.nb[j] = nmn[j]; F.dext[j] = dmn[j]; F.pext[j] = pr; }
+      if (pos_(pr)) {
+        const R t = div_(dmx[j], pr);
+        if (less_(t, F.alRaw[j])) { F.alRaw[j] = t; F.side[j] = 1; F.face[j] = e; F.nb[j] = nmx[j]; F.dext[j] = dmx[j]; F.pext[j] = pr; }
+      } else if (neg_(pr)) {
+        const R t = div_(dmn[j], pr);
+        if (less_(t, F.alRaw[j])) { F.alRaw[j] = t; F.side[j] = 2; F.face[j] = e; F.nb[j] = nmn[j]; F.dext[j] = dmn[j]; F.pext[j] = pr; }
       }
     }
   }
@@ -604,8 +604,8 @@ __device__ inline void velFrameReverse(const View<R> &V, const L &ld, int i, con
   for (int j = 0; j < 3; ++j) {
     if (F.side[j] == 0 || F.held[j] || albRaw[j] == R(0)) continue;
     // alRaw = dext / pr: the same guarded form as the scalar limiter's
-    const R r = albRaw[j] / F.pext[j];
-    const R dextb = r, prb = -r * (F.dext[j] / F.pext[j]);
+    const R r = div_(albRaw[j], F.pext[j]);
+    const R dextb = r, prb = -r * div_(F.dext[j], F.pext[j]);
     if (F.nb[j] >= 0) {
       R un[4];
       ld.prim4(F.nb[j], un);
@@ -668,7 +668,7 @@ __device__ inline void velFrameReverse(const View<R> &V, const L &ld, int i, con
         ajk += Ab[a + 3 * j] * A[a + 3 * k];
         akj += Ab[a + 3 * k] * A[a + 3 * j];
       }
-      const R coef = (ajk - akj) / (F.ev[j] - F.ev[k]);
+      const R coef = div_(ajk - akj, F.ev[j] - F.ev[k]);
 #pragma unroll
       for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -804,8 +804,8 @@ __global__ void __launch_bounds__(kBlock) kAdjGradFwd(View<R> V, AdjWork<R> W, c
       }
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
-        if (x[k] < vmin[k]) { vmin[k] = x[k]; jmin[k] = nb; }
-        if (x[k] > vmax[k]) { vmax[k] = x[k]; jmax[k] = nb; }
+        if (less_(x[k], vmin[k])) { vmin[k] = x[k]; jmin[k] = nb; }
+        if (less_(vmax[k], x[k])) { vmax[k] = x[k]; jmax[k] = nb; }
       }
     }
     const R epsq = V.epsq[i];
@@ -817,8 +817,8 @@ __global__ void __launch_bounds__(kBlock) kAdjGradFwd(View<R> V, AdjWork<R> W, c
       for (int k = 0; k < 5; ++k) {
         if (rc == 10 && k >= 1 && k <= 3) continue;  // the eigen-frame limiter below
         const R d2 = -(g[3 * k] * d[0] + g[3 * k + 1] * d[1] + g[3 * k + 2] * d[2]);
-        if (!(d2 > R(0)) && !(d2 < R(0))) continue;
-        const bool up = d2 > R(0);
+        const bool up = pos_(d2);
+        if (!up && !neg_(d2)) continue;
         const R dext = up ? vmax[k] - q[k] : vmin[k] - q[k];
         R t;
         bool active;
@@ -826,11 +826,11 @@ __global__ void __launch_bounds__(kBlock) kAdjGradFwd(View<R> V, AdjWork<R> W, c
           t = venkat(dext, d2, epsq);
           active = true;
         } else {
-          const R x = dext / d2;
+          const R x = div_(dext, d2);
           t = fmin2(R(1), x);
-          active = x < R(1);
+          active = less_(x, R(1));
         }
-        if (t < lim[k]) {
+        if (less_(t, lim[k])) {
           lim[k] = t;
           es[k] = active ? e : -1;
           js[k] = up ? jmax[k] : jmin[k];
@@ -947,7 +947,7 @@ __global__ void __launch_bounds__(kBlock) kAdjWenoFwdLanes(View<R> V, AdjWork<R>
     if (xyz) {
 #pragma unroll
       for (int k = 0; k < 15; ++k) {
-        const R w = h == 0 ? R(1) / (own[k] * own[k] + eps) : R(0);
+        const R w = h == 0 ? div_(R(1), own[k] * own[k] + eps) : R(0);
         sum[k] = w;
         g[k] = w * own[k];
       }
@@ -955,7 +955,7 @@ __global__ void __launch_bounds__(kBlock) kAdjWenoFwdLanes(View<R> V, AdjWork<R>
         fetch(s);
 #pragma unroll
         for (int k = 0; k < 15; ++k) {
-          const R w = R(1) / (t[k] * t[k] + eps);
+          const R w = div_(R(1), t[k] * t[k] + eps);
           sum[k] = sum[k] + w;
           g[k] = g[k] + w * t[k];
         }
@@ -963,13 +963,13 @@ __global__ void __launch_bounds__(kBlock) kAdjWenoFwdLanes(View<R> V, AdjWork<R>
       join(sum, 15);
       join(g, 15);
 #pragma unroll
-      for (int k = 0; k < 15; ++k) g[k] = g[k] / sum[k];
+      for (int k = 0; k < 15; ++k) g[k] = div_(g[k], sum[k]);
     } else {
       R w0[5];
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
         const R m = fabs_(own[3 * v]) + fabs_(own[3 * v + 1]) + fabs_(own[3 * v + 2]);
-        w0[v] = R(1) / (m * m + eps);
+        w0[v] = div_(R(1), m * m + eps);
         sum[v] = h == 0 ? w0[v] : R(0);
       }
       for (int s = sb + h; s < se; s += kL) {
@@ -977,13 +977,13 @@ __global__ void __launch_bounds__(kBlock) kAdjWenoFwdLanes(View<R> V, AdjWork<R>
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
           const R m = fabs_(t[3 * v]) + fabs_(t[3 * v + 1]) + fabs_(t[3 * v + 2]);
-          sum[v] = sum[v] + R(1) / (m * m + eps);
+          sum[v] = sum[v] + div_(R(1), m * m + eps);
         }
       }
       join(sum, 5);
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
-        const R term = h == 0 ? w0[v] / sum[v] : R(0);
+        const R term = h == 0 ? div_(w0[v], sum[v]) : R(0);
 #pragma unroll
         for (int d = 0; d < 3; ++d) g[3 * v + d] = term * own[3 * v + d];
       }
@@ -992,7 +992,7 @@ __global__ void __launch_bounds__(kBlock) kAdjWenoFwdLanes(View<R> V, AdjWork<R>
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
           const R m = fabs_(t[3 * v]) + fabs_(t[3 * v + 1]) + fabs_(t[3 * v + 2]);
-          const R term = (R(1) / (m * m + eps)) / sum[v];
+          const R term = div_(div_(R(1), m * m + eps), sum[v]);
 #pragma unroll
           for (int d = 0; d < 3; ++d) g[3 * v + d] = g[3 * v + d] + term * t[3 * v + d];
         }
@@ -1300,7 +1300,7 @@ __global__ void __launch_bounds__(kBlock) kAdjCell1(View<R> V, AdjWork<R> W) {
     }
   }
   // irl = 1/rho of the cell (HLLC: Hl = el + irl*pl)
-  qb[0] += rbar * (R(-1) / (rho * rho));
+  qb[0] += rbar * div_(R(-1), rho * rho);
   R gb[15], nbb[5] = {0, 0, 0, 0, 0};
   int nbt[5] = {-1, -1, -1, -1, -1};  // the neighbour receiving nbb[k]
 #pragma unroll
@@ -1350,9 +1350,9 @@ __global__ void __launch_bounds__(kBlock) kAdjCell1(View<R> V, AdjWork<R> W) {
         // as (lb/d2) and -(lb/d2)*(dext/d2) so that a tiny d2 (differences of
         // ~1e-200 ahead of a wave) neither squares into 0 nor makes 0/0 at a
         // local extreme (dext = 0)
-        const R r = lb / d2;
+        const R r = div_(lb, d2);
         db = r;
-        d2b = -r * (dext / d2);
+        d2b = -r * div_(dext, d2);
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) gb[3 * k + c] += d2b * (-dxyz[c]);
@@ -1407,7 +1407,7 @@ __global__ void __launch_bounds__(kBlock) kAdjCell1(View<R> V, AdjWork<R> W) {
 #pragma unroll
     for (int k = 0; k < 15; ++k) sw[k] = W.gradd[(rc == 2 ? k : k / 3) * n + i];
 #pragma unroll
-    for (int k = 0; k < 15; ++k) a[k] = gb[k] / sw[k];
+    for (int k = 0; k < 15; ++k) a[k] = div_(gb[k], sw[k]);
     if constexpr (Layout<R>::packed) storeGradTo(V, V.gradRaw, i, a);
     else storeGradTo(V, W.gradd, i, a);
   }
@@ -1523,7 +1523,7 @@ __global__ void __launch_bounds__(kBlock) kAdjWeno(View<R> V, AdjWork<R> W) {
     if (xyz) {
 #pragma unroll
       for (int k = 0; k < 15; ++k) {
-        const R w = R(1) / (tt[k] * tt[k] + eps);
+        const R w = div_(R(1), tt[k] * tt[k] + eps);
         const R wp = R(-2) * tt[k] * w * w;
         out[k] = (w + wp * tt[k]) * a[k] - wp * ag[k];
       }
@@ -1532,7 +1532,7 @@ __global__ void __launch_bounds__(kBlock) kAdjWeno(View<R> V, AdjWork<R> W) {
       for (int v = 0; v < 5; ++v) {
         const R *tv = tt + 3 * v, *av = a + 3 * v, *bv = ag + 3 * v;
         const R T = fabs_(tv[0]) + fabs_(tv[1]) + fabs_(tv[2]);
-        const R w = R(1) / (T * T + eps);
+        const R w = div_(R(1), T * T + eps);
         const R c = R(-2) * T * w * w * (tv[0] * av[0] + tv[1] * av[1] + tv[2] * av[2] - (bv[0] + bv[1] + bv[2]));
 #pragma unroll
         for (int d = 0; d < 3; ++d) out[3 * v + d] = w * av[d] + (tv[d] < R(0) ? -c : c);
@@ -1680,10 +1680,10 @@ __global__ void __launch_bounds__(kBlock) kAdjCell2(View<R> V, AdjWork<R> W, dou
         const int r = rk >> 3, k = rk & 7, b = V.cRowFace[r];
         const double *K = V.patchK + kPatchK * V.bpatch[b];
         const double rt = rgas * K[1];
-        double dval = 1.0 / rt;  // d rho / dp
+        double dval = div_(1.0, rt);  // d rho / dp
         if (k > 0) {
-          const double rl = p / rt, nk = (k == 1) ? V.bnx[b] : (k == 2) ? V.bny[b] : V.bnz[b];
-          dval = K[0] * nk / (rl * rl) * dval;
+          const double rl = div_(p, rt), nk = (k == 1) ? V.bnx[b] : (k == 2) ? V.bny[b] : V.bnz[b];
+          dval = div_(K[0] * nk, rl * rl) * dval;
         }
         const R dot = V.cW[3 * (size_t)r] * W.Gbar[(3 * k) * n + i] + V.cW[3 * (size_t)r + 1] * W.Gbar[(3 * k + 1) * n + i] +
                       V.cW[3 * (size_t)r + 2] * W.Gbar[(3 * k + 2) * n + i];

@@ -22,6 +22,7 @@
 #include "constr.h"
 #include "ctx.h"
 #include "errors.h"
+#include "intmath.h"
 #include "fixedsum.h"
 #include "ops.h"
 #include "tiles.h"
@@ -170,8 +171,8 @@ ArgMem pointerKind(const void *p, int *device) {
 
 // FP64 FMA throughput probe: 8 independent chains per thread.
 __device__ double gFmaSink;
-// Self-check of f2d/d2f against the hardware conversions.  Value k of the
-// sample: a 64-bit hash of (seed, k); by k mod 4 its bits as a double, a
+// Self-check of f2d/d2f and of the integer pipe's division, square root and
+// comparisons (intmath.h) against the hardware's.  Value k of the sample: a 64-bit hash of (seed, k); by k mod 4 its bits as a double, a
 // double with an exponent near the float range (normal, denormal and
 // overflowing results), the same with the 29 bits dropped by the rounding set
 // to a tie, or a float (its hash bits) widened, plus the midpoint between it
@@ -190,6 +191,23 @@ __global__ void kCvtCheck(long long n, unsigned long long seed, unsigned long lo
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
     const unsigned long long h = mix64(seed ^ mix64((unsigned long long)k));
     const int mode = (int)(k & 3);
+    {
+      // a any bits, b any bits (mode 0) or an exponent near a's, every fourth
+      // a short significand (exact and nearly half-way results)
+      const unsigned long long h2 = mix64(h);
+      const unsigned long long cut = mode == 3 ? ~0ull << (h % 52) : ~0ull;
+      const double a = __longlong_as_double((long long)(h & (cut | 0xFFF0000000000000ull)));
+      const unsigned long long near = (h & 0x7FF0000000000000ull) + (((h2 >> 52) & 7ull) << 52);
+      const double b = __longlong_as_double(
+          (long long)(mode == 0 ? h2 : ((h2 & 0x800FFFFFFFFFFFFFull) | (near & 0x7FF0000000000000ull))));
+      auto same = [](double x, double y) {
+        return __double_as_longlong(x) == __double_as_longlong(y) || (isnan(x) && isnan(y));
+      };
+      if (!same(intDiv(a, b), __ddiv_rn(a, b)) || !same(intSqrt(fabs(a)), __dsqrt_rn(fabs(a))) ||
+          isLess(a, b) != (a < b) || isLessEq(a, b) != (a <= b) || isLess(b, b) || isPos(a) != (a > 0.0) ||
+          isNeg(a) != (a < 0.0))
+        ++miss;
+    }
     if (mode < 3) {
       unsigned long long bits = h;
       if (mode >= 1) {

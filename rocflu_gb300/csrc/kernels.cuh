@@ -71,12 +71,12 @@ __device__ inline void dependentVars(const Params &p, const double *cv, double &
   const double gc = p.gcR;  // MixtPerf_R_M(gv(GV_MIXT_MOL)), computed once
   const double g = p.gRT;   // MixtPerf_G_CpR(gv(GV_MIXT_CP), gc)
   double r = cv[0];
-  double ir = 1.0 / r;
+  double ir = div_(1.0, r);
   double Eo = ir * cv[4];
   double Vm2 = ir * ir * (cv[1] * cv[1] + cv[2] * cv[2] + cv[3] * cv[3]);
   pres = (g - 1.0) * r * (Eo - 0.5 * Vm2);
-  temp = pres / (r * gc);
-  snd = sqrt(g * gc * temp);
+  temp = div_(pres, r * gc);
+  snd = sqrt_(g * gc * temp);
 }
 
 template <typename R>
@@ -340,7 +340,7 @@ struct MixedPrim {
 // (modflu/RFLU_ModConvertCv.F90:214-224)
 template <typename R>
 __device__ inline void storePrim(const View<R> &V, int i, const double *cv, double pres) {
-  double ir = 1.0 / cv[0];
+  double ir = div_(1.0, cv[0]);
   storePrimRec(V, i, (R)cv[0], (R)(ir * cv[1]), (R)(ir * cv[2]), (R)(ir * cv[3]), (R)pres);
 }
 
@@ -414,9 +414,9 @@ __device__ inline S constrValue(const View<R> &V, const L &ld, int b, int k) {
   const S rgas = S(8314.3) / S(V.p.gvMol);
   // the face's cell pressure through the loader (the tangent's carries its
   // derivative)
-  const S rl = S(ld.dv(0, V.bcell[b])) / (rgas * S(K[1]));  // MixtPerf_D_PRT(pl, rGas, tInj)
+  const S rl = div_(S(ld.dv(0, V.bcell[b])), rgas * S(K[1]));  // MixtPerf_D_PRT(pl, rGas, tInj)
   if (k == 0) return rl;
-  const S ql = -S(K[0]) / rl + S(0);
+  const S ql = div_(-S(K[0]), rl) + S(0);
   return ql * n;
 }
 
@@ -533,7 +533,7 @@ __device__ inline void reflectGrad(const Qt *Q, S *g) {
 // cell instead of once per (cell, member) pair.
 template <typename R>
 __device__ inline void storeWenoWeight(const View<R> &V, int k, int i, R t) {
-  V.wenoW[(size_t)k * V.nc + i] = R(1) / (t * t + R(1.0e-15));
+  V.wenoW[(size_t)k * V.nc + i] = div_(R(1), t * t + R(1.0e-15));
 }
 
 // Gradient + limiter of one cell.
@@ -600,7 +600,7 @@ __device__ inline void gradLimitCell(const View<R> &V, const L &ld, int i, typen
           reflect3(V.xfQ + 9 * V.stXf[s], u, qj + 1);
         }
       }
-      const S inv = S(1) / (dx * dx + dy * dy + dz * dz);
+      const S inv = div_(S(1), dx * dx + dy * dy + dz * dz);
       const S sx = inv * dx, sy = inv * dy, sz = inv * dz;
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
@@ -685,22 +685,22 @@ __device__ inline void limitCell(const View<R> &V, const L &ld, int i, const typ
         S d2 = -(g[3 * k] * dx + g[3 * k + 1] * dy + g[3 * k + 2] * dz);
         S dmax = vmax[k] - q[k], dmin = vmin[k] - q[k];
         if (kOnePass && rc != 11) {
-          if (d2 > S(0)) pmx[k] = fmax2(pmx[k], d2);
-          else if (d2 < S(0)) nmn[k] = fmin2(nmn[k], d2);
+          if (pos_(d2)) pmx[k] = fmax2(pmx[k], d2);
+          else if (neg_(d2)) nmn[k] = fmin2(nmn[k], d2);
         } else if (rc == 11) {
           const S tiny = S(1.0e-12);
-          if (d2 > S(0)) {
+          if (pos_(d2)) {
             S numer = (dmax * dmax + epsq) * d2 + S(2) * d2 * d2 * dmax;
             S denom = d2 * (dmax * dmax + S(2) * d2 * d2 + dmax * d2 + epsq);
-            lim[k] = fmin2(numer / (denom + tiny), lim[k]);
-          } else if (d2 < S(0)) {
+            lim[k] = fmin2(div_(numer, denom + tiny), lim[k]);
+          } else if (neg_(d2)) {
             S numer = (dmin * dmin + epsq) * d2 + S(2) * d2 * d2 * dmin;
             S denom = d2 * (dmin * dmin + S(2) * d2 * d2 + dmin * d2 + epsq);
-            lim[k] = fmin2(numer / (denom + tiny), lim[k]);
+            lim[k] = fmin2(div_(numer, denom + tiny), lim[k]);
           }
         } else {
-          if (d2 > S(0)) lim[k] = fmin2(fmin2(S(1), dmax / d2), lim[k]);
-          else if (d2 < S(0)) lim[k] = fmin2(fmin2(S(1), dmin / d2), lim[k]);
+          if (pos_(d2)) lim[k] = fmin2(fmin2(S(1), div_(dmax, d2)), lim[k]);
+          else if (neg_(d2)) lim[k] = fmin2(fmin2(S(1), div_(dmin, d2)), lim[k]);
         }
       }
     }
@@ -709,8 +709,8 @@ __device__ inline void limitCell(const View<R> &V, const L &ld, int i, const typ
       for (int k = 0; k < 5; ++k) {
         if (rc == 10 && k >= 1 && k <= 3) continue;
         const S dmax = vmax[k] - q[k], dmin = vmin[k] - q[k];
-        if (pmx[k] > S(0)) lim[k] = fmin2(fmin2(S(1), dmax / pmx[k]), lim[k]);
-        if (nmn[k] < S(0)) lim[k] = fmin2(fmin2(S(1), dmin / nmn[k]), lim[k]);
+        if (pos_(pmx[k])) lim[k] = fmin2(fmin2(S(1), div_(dmax, pmx[k])), lim[k]);
+        if (neg_(nmn[k])) lim[k] = fmin2(fmin2(S(1), div_(dmin, nmn[k])), lim[k]);
       }
     }
     if (rc == 10) {
@@ -782,19 +782,19 @@ __device__ inline void limitCell(const View<R> &V, const L &ld, int i, const typ
           pr = pr + A[3 * j + 1] * sh[1];
           pr = pr + A[3 * j + 2] * sh[2];
           if (kOnePass) {
-            if (pr > S(0)) spx[j] = fmax2(spx[j], pr);
-            else if (pr < S(0)) snx[j] = fmin2(snx[j], pr);
+            if (pos_(pr)) spx[j] = fmax2(spx[j], pr);
+            else if (neg_(pr)) snx[j] = fmin2(snx[j], pr);
           } else {
-            if (pr > S(0)) al[j] = fmin2(al[j], dmx[j] / pr);
-            else if (pr < S(0)) al[j] = fmin2(al[j], dmn[j] / pr);
+            if (pos_(pr)) al[j] = fmin2(al[j], div_(dmx[j], pr));
+            else if (neg_(pr)) al[j] = fmin2(al[j], div_(dmn[j], pr));
           }
         }
       }
       if (kOnePass) {
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-          if (spx[j] > S(0)) al[j] = fmin2(al[j], dmx[j] / spx[j]);
-          if (snx[j] < S(0)) al[j] = fmin2(al[j], dmn[j] / snx[j]);
+          if (pos_(spx[j])) al[j] = fmin2(al[j], div_(dmx[j], spx[j]));
+          if (neg_(snx[j])) al[j] = fmin2(al[j], div_(dmn[j], snx[j]));
         }
       }
       holdIdleAxes(A, G, al);
@@ -802,7 +802,7 @@ __device__ inline void limitCell(const View<R> &V, const L &ld, int i, const typ
       mx = fmax2(mx, fabs_(ev[1]));
       mx = fmax2(mx, fabs_(ev[2]));
       const S scale = S(1.0e-3) * mx;
-      const bool e12 = (ev[1] - ev[0] <= scale), e23 = (ev[2] - ev[1] <= scale);
+      const bool e12 = lessEq_(ev[1] - ev[0], scale), e23 = lessEq_(ev[2] - ev[1], scale);
       if (e12 && e23) {
         S m = fmin2(fmin2(al[0], al[1]), al[2]);
         al[0] = al[1] = al[2] = m;
@@ -1910,7 +1910,7 @@ __device__ inline void wenoXyz(const R *own, int sb, int se, Fetch fetch, R *g, 
   const R eps = R(1.0e-15);
 #pragma unroll
   for (int k = 0; k < 15; ++k) {
-    sum[k] = R(1) / (own[k] * own[k] + eps);
+    sum[k] = div_(R(1), own[k] * own[k] + eps);
     g[k] = sum[k] * own[k];
   }
   for (int s = sb; s < se; ++s) {
@@ -1918,13 +1918,13 @@ __device__ inline void wenoXyz(const R *own, int sb, int se, Fetch fetch, R *g, 
     fetch(s, t);
 #pragma unroll
     for (int k = 0; k < 15; ++k) {
-      const R w = R(1) / (t[k] * t[k] + eps);
+      const R w = div_(R(1), t[k] * t[k] + eps);
       sum[k] = sum[k] + w;
       g[k] = g[k] + w * t[k];
     }
   }
 #pragma unroll
-  for (int k = 0; k < 15; ++k) g[k] = g[k] / sum[k];
+  for (int k = 0; k < 15; ++k) g[k] = div_(g[k], sum[k]);
 }
 template <typename R, typename Fetch>
 __device__ inline void wenoXyz(const R *own, int sb, int se, Fetch fetch, R *g) {
@@ -1941,7 +1941,7 @@ __device__ inline void wenoSimple(const R *own, int sb, int se, Fetch fetch, R *
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
     const R t = fabs_(own[3 * v]) + fabs_(own[3 * v + 1]) + fabs_(own[3 * v + 2]);
-    w0[v] = R(1) / (t * t + eps);
+    w0[v] = div_(R(1), t * t + eps);
     sum[v] = w0[v];
   }
   for (int s = sb; s < se; ++s) {
@@ -1950,12 +1950,12 @@ __device__ inline void wenoSimple(const R *own, int sb, int se, Fetch fetch, R *
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
       const R m = fabs_(t[3 * v]) + fabs_(t[3 * v + 1]) + fabs_(t[3 * v + 2]);
-      sum[v] = sum[v] + R(1) / (m * m + eps);
+      sum[v] = sum[v] + div_(R(1), m * m + eps);
     }
   }
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
-    const R term = w0[v] / sum[v];
+    const R term = div_(w0[v], sum[v]);
 #pragma unroll
     for (int d = 0; d < 3; ++d) g[3 * v + d] = term * own[3 * v + d];
   }
@@ -1965,7 +1965,7 @@ __device__ inline void wenoSimple(const R *own, int sb, int se, Fetch fetch, R *
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
       const R m = fabs_(t[3 * v]) + fabs_(t[3 * v + 1]) + fabs_(t[3 * v + 2]);
-      const R term = (R(1) / (m * m + eps)) / sum[v];
+      const R term = div_(div_(R(1), m * m + eps), sum[v]);
 #pragma unroll
       for (int d = 0; d < 3; ++d) g[3 * v + d] = g[3 * v + d] + term * t[3 * v + d];
     }
@@ -1985,8 +1985,8 @@ __device__ inline int simplePositivity(R q0, R q4, int nFaces, Face face, R *g) 
   for (int k = 0; k < nFaces; ++k) {
     R d[3];
     if (!face(k, d)) continue;
-    if (q0 + g[0] * d[0] + g[1] * d[1] + g[2] * d[2] <= R(0)) z0 = true;
-    if (q4 + g[12] * d[0] + g[13] * d[1] + g[14] * d[2] <= R(0)) z4 = true;
+    if (lessEq_(q0 + g[0] * d[0] + g[1] * d[1] + g[2] * d[2], R(0))) z0 = true;
+    if (lessEq_(q4 + g[12] * d[0] + g[13] * d[1] + g[14] * d[2], R(0))) z4 = true;
   }
   if (z0) g[0] = g[1] = g[2] = R(0);
   if (z4) g[12] = g[13] = g[14] = R(0);
@@ -2049,22 +2049,29 @@ __global__ void __launch_bounds__(kBlock) kWenoSmooth(View<R> V, const R *raw) {
 // one more); the sums run in the same order with the same operations, so the
 // results are the same bits.  A member seen reflected across symmetry patches
 // is another gradient: its weight is formed here, as are all of them where the
-// view holds none (rflu_gpu_residual_static).  Bound by the FP64 pipe.
+// view holds none (kStored false, rflu_gpu_residual_static).  Bound by the
+// FP64 pipe.
 // Measured with kGradVar: 20 FP64_EXACT steps of 512 cells 13.1 -> 3.7 ms, 2
 // FP64 steps of a periodic 40^3 box 3.73 -> 2.56 ms.
-template <typename R>
+// a b + c: one rounding in RFLU_PREC_FP64, two in FP64_EXACT.  Spelled out where
+// the compiler moved the addition behind a branch and left the product on both
+// sides of it (a third FP64 instruction per member: 125 -> 170 us).
+__device__ inline double mulAdd(double a, double b, double c) {
+  return kFixedSums ? __fma_rn(a, b, c) : __dadd_rn(c, __dmul_rn(a, b));
+}
+template <typename R, bool kStored>
 __global__ void __launch_bounds__(kBlock) kWenoVar(View<R> V, const R *raw) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const int v = blockIdx.y;
   const size_t n = V.nc, nb = V.nb;
-  const R *w = V.wenoW ? V.wenoW + 3 * v * n : nullptr, *t = raw + 3 * v * n;
-  auto weight = [](R tc) { return R(1) / (tc * tc + R(1.0e-15)); };
+  const R *w = kStored ? V.wenoW + 3 * v * n : nullptr, *t = raw + 3 * v * n;
+  auto weight = [](R tc) { return div_(R(1), tc * tc + R(1.0e-15)); };
   R sum[3], g[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const R tc = t[c * n + i];
-    sum[c] = w ? w[c * n + i] : weight(tc);
+    sum[c] = kStored ? w[c * n + i] : weight(tc);
     g[c] = __dmul_rn(sum[c], tc);  // rounded by itself, whatever the loop below is compiled to
   }
   const int se = V.stOff[i + 1];
@@ -2082,20 +2089,20 @@ __global__ void __launch_bounds__(kBlock) kWenoVar(View<R> V, const R *raw) {
         const R tc = v == 0 ? tr[c] : v == 1 ? tr[3 + c] : v == 2 ? tr[6 + c] : v == 3 ? tr[9 + c] : tr[12 + c];
         const R ww = weight(tc);
         sum[c] = sum[c] + ww;
-        g[c] = g[c] + ww * tc;
+        g[c] = mulAdd(ww, tc, g[c]);
       }
     } else {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const R tc = t[c * n + j];
-        const R ww = w ? w[c * n + j] : weight(tc);
+        const R ww = kStored ? w[c * n + j] : weight(tc);
         sum[c] = sum[c] + ww;
-        g[c] = g[c] + ww * tc;
+        g[c] = mulAdd(ww, tc, g[c]);
       }
     }
   }
 #pragma unroll
-  for (int c = 0; c < 3; ++c) g[c] = g[c] / sum[c];
+  for (int c = 0; c < 3; ++c) g[c] = div_(g[c], sum[c]);
   if (v == 0 || v == 4) {
     const R q = V.prim[v * n + i];
     bool zero = false;
@@ -2110,7 +2117,7 @@ __global__ void __launch_bounds__(kBlock) kWenoVar(View<R> V, const R *raw) {
         d[1] = V.bd[nb + b];
         d[2] = V.bd[2 * nb + b];
       }
-      if (q + g[0] * d[0] + g[1] * d[1] + g[2] * d[2] <= R(0)) zero = true;
+      if (lessEq_(q + g[0] * d[0] + g[1] * d[1] + g[2] * d[2], R(0))) zero = true;
     }
     if (zero) g[0] = g[1] = g[2] = R(0);
   }
@@ -2281,7 +2288,7 @@ __device__ inline void faceState(const View<R> &V, const L &ld, int c, typename 
   ld.prim5(c, q);
   ld.grad15(c, gr);
   S r = q[0];
-  S ir = S(1) / r;
+  S ir = div_(S(1), r);
   S u = q[1], v = q[2], w = q[3];
   if (Ref<R>::on) {
     // ul = pCv(CV_MIXT_XMOM,c1)*irl with pCv(XMOM) = r*u after RFLU_ConvertCvPrim2Cons
@@ -2306,20 +2313,20 @@ template <typename S>
 __device__ inline void riemann2(const Params &P, S nx, S ny, S nz, S nm, const S *L, S irl, const S *Rt, S irr, S *flx) {
   const S cp = prm<S>(P.refCp, P.refCpF), g = prm<S>(P.refGamma, P.refGammaF);
   if (P.spaceDiscr == 1) {
-    S gc = cp - cp / g;
-    S tl = L[4] / (L[0] * gc), tr = Rt[4] / (Rt[0] * gc);
+    S gc = cp - div_(cp, g);
+    S tl = div_(L[4], L[0] * gc), tr = div_(Rt[4], Rt[0] * gc);
     S Hl = perfHo(cp, tl, L[1], L[2], L[3]), Hr = perfHo(cp, tr, Rt[1], Rt[2], Rt[3]);
     roeFlux(g, prm<S>(P.epsEntr, P.epsEntrF), prm<S>(P.dissFact, P.dissFactF), nx, ny, nz, nm, L[0], L[1], L[2], L[3],
             L[4], Hl, Rt[0], Rt[1], Rt[2], Rt[3], Rt[4], Hr, flx);
   } else if (P.spaceDiscr == 3) {
-    S el = perfEo(L[0], g, L[4], L[1], L[2], L[3]), al = sqrt_(g * L[4] / L[0]);
-    S er = perfEo(Rt[0], g, Rt[4], Rt[1], Rt[2], Rt[3]), ar = sqrt_(g * Rt[4] / Rt[0]);
+    S el = perfEo(L[0], g, L[4], L[1], L[2], L[3]), al = sqrt_(div_(g * L[4], L[0]));
+    S er = perfEo(Rt[0], g, Rt[4], Rt[1], Rt[2], Rt[3]), ar = sqrt_(div_(g * Rt[4], Rt[0]));
     S Hl = el + irl * L[4], Hr = er + irr * Rt[4];
     hllcFlux(g, nx, ny, nz, nm, L[0], L[1], L[2], L[3], L[4], el, al, Hl, Rt[0], Rt[1], Rt[2], Rt[3], Rt[4], er, ar,
              Hr, flx);
   } else {
-    S gc = cp - cp / g;
-    S tl = L[4] / (L[0] * gc), tr = Rt[4] / (Rt[0] * gc);
+    S gc = cp - div_(cp, g);
+    S tl = div_(L[4], L[0] * gc), tr = div_(Rt[4], Rt[0] * gc);
     S al = sqrt_(g * gc * tl), ar = sqrt_(g * gc * tr);
     S Hl = perfHo(cp, tl, L[1], L[2], L[3]), Hr = perfHo(cp, tr, Rt[1], Rt[2], Rt[3]);
     ausmFlux(nx, ny, nz, nm, L[0], L[1], L[2], L[3], L[4], Hl, al, Rt[0], Rt[1], Rt[2], Rt[3], Rt[4], Hr, ar, flx);
@@ -2330,8 +2337,8 @@ __device__ inline void riemann2(const Params &P, S nx, S ny, S nz, S nm, const S
 template <typename H>
 __device__ inline void riemann1(const Params &P, const H *cl, const H *dvl, const H *cr, const H *dvr, H nx, H ny,
                                 H nz, H nm, H *flx) {
-  H rl = cl[0], irl = H(1) / rl, ul = cl[1] * irl, vl = cl[2] * irl, wl = cl[3] * irl;
-  H rr = cr[0], irr = H(1) / rr, ur = cr[1] * irr, vr = cr[2] * irr, wr = cr[3] * irr;
+  H rl = cl[0], irl = div_(H(1), rl), ul = cl[1] * irl, vl = cl[2] * irl, wl = cl[3] * irl;
+  H rr = cr[0], irr = div_(H(1), rr), ur = cr[1] * irr, vr = cr[2] * irr, wr = cr[3] * irr;
   H pl = dvl[0], pr = dvr[0];
   const H cp = H(P.refCp), g = H(P.refGamma);
   if (P.spaceDiscr == 1) {
@@ -2342,7 +2349,7 @@ __device__ inline void riemann1(const Params &P, const H *cl, const H *dvl, cons
     H Hl = el + irl * pl, Hr = er + irr * pr;
     hllcFlux(g, nx, ny, nz, nm, rl, ul, vl, wl, pl, el, dvl[2], Hl, rr, ur, vr, wr, pr, er, dvr[2], Hr, flx);
   } else {
-    H Hl = cl[4] * irl + pl / rl, Hr = cr[4] * irr + pr / rr;
+    H Hl = cl[4] * irl + div_(pl, rl), Hr = cr[4] * irr + div_(pr, rr);
     ausmFlux(nx, ny, nz, nm, rl, ul, vl, wl, pl, Hl, dvl[2], rr, ur, vr, wr, pr, Hr, dvr[2], flx);
   }
 }
@@ -2361,7 +2368,7 @@ __device__ inline void patch1(const Params &P, int type, int bcOpt, const double
 #pragma unroll
   for (int k = 0; k < 5; ++k) cv[k] = cvIn[k];
   if (P.spaceOrder == 2) {
-    const H ir = H(1) / cv[0];
+    const H ir = div_(H(1), cv[0]);
     const H up = ir * cv[1], vp = ir * cv[2], wp = ir * cv[3];
     cv[1] = cv[0] * up;
     cv[2] = cv[0] * vp;
@@ -2387,7 +2394,7 @@ __device__ inline void patch1(const Params &P, int type, int bcOpt, const double
     return;
   }
   const H cp = H(P.gvCp), rgas = H(8314.3) / H(P.gvMol);
-  const H g = cp / (cp - rgas);
+  const H g = div_(cp, cp - rgas);
   if (type == 90) {
     injectionPatchFlux(K, g, cp, rgas, nx, ny, nz, nm, cv[0], cv[1], cv[2], cv[3], pl, fd);
     return;
@@ -2415,8 +2422,8 @@ __device__ inline void patch2(const Params &P, int type, int bcOpt, const double
     return;
   }
   const S cp = prm<S>(P.gvCp, P.gvCpF), mol = prm<S>(P.gvMol, P.gvMolF);
-  S rgas = S(8314.3) / mol;
-  S g = cp / (cp - rgas);
+  S rgas = div_(S(8314.3), mol);
+  S g = div_(cp, cp - rgas);
   S rul = L[0] * L[1], rvl = L[0] * L[2], rwl = L[0] * L[3];
   if (type == 90) {
     injectionPatchFlux(K, g, cp, rgas, nx, ny, nz, nm, L[0], rul, rvl, rwl, L[4], flx);
@@ -2609,27 +2616,27 @@ template <typename R>
 __device__ inline void afterUpdate(const View<R> &V, int i, double *cv, double &pr, double &tp, double &cs) {
   const Params &P = V.p;
   {
-    double rho = cv[0], rrho = 1.0 / rho;
+    double rho = cv[0], rrho = div_(1.0, rho);
     double u = rrho * cv[1], v = rrho * cv[2], w = rrho * cv[3];
-    if (isnan(rho) || isnan(u) || isnan(v) || isnan(w) || isnan(pr) || isnan(tp)) {
+    if (isNan_(rho) || isNan_(u) || isNan_(v) || isNan_(w) || isNan_(pr) || isNan_(tp)) {
       atomicAdd(&V.sc->nanCells, 1ull);
       atomicMin(&V.sc->firstBadCell, V.refId[i] + 1);
     }
   }
   const double gamma = P.gRT;
   {
-    double r = cv[0], ir = 1.0 / r;
+    double r = cv[0], ir = div_(1.0, r);
     double u = ir * cv[1], v = ir * cv[2], w = ir * cv[3];
     double Eo = ir * cv[4];
     double Vm2 = u * u + v * v + w * w;
     double p = (gamma - 1.0) * r * (Eo - 0.5 * Vm2);
-    if (p <= 0.0 && fabs(p) <= 1.0e-12) {
+    if (lessEq_(p, 0.0) && fabs(p) <= 1.0e-12) {
       atomicAdd(&V.sc->negPCells, 1ull);
       cv[4] = r * perfEo(r, gamma, 1.0e-12, u, v, w);
     }
   }
-  if (pr <= 0.0) {
-    double rho = cv[0], rrho = 1.0 / rho;
+  if (lessEq_(pr, 0.0)) {
+    double rho = cv[0], rrho = div_(1.0, rho);
     double u = rrho * cv[1], v = rrho * cv[2], w = rrho * cv[3];
     double Vm2 = u * u + v * v + w * w;
     atomicAdd(&V.sc->posFixCells, 1ull);
@@ -2707,7 +2714,7 @@ __device__ inline void mixedUpdate(const View<R> &V, int i, int iStage, float fa
     atomicAdd(&V.sc->nanCells, 1ull);
     atomicMin(&V.sc->firstBadCell, V.refId[i] + 1);
   }
-  if (pr <= 0.0) {
+  if (lessEq_(pr, 0.0)) {
     if (fabs(pr) <= 1.0e-12) atomicAdd(&V.sc->negPCells, 1ull);
     atomicAdd(&V.sc->posFixCells, 1ull);
     cv[4] = 1.0e4 * cv[0] + ke;
@@ -2749,7 +2756,7 @@ __global__ void __launch_bounds__(kBlock) kGatherUpdate(View<R> V, int iStage, c
   }
   const double fac = P.ark[iStage - 1] * (*dtp);
   const double grk = P.grk[iStage - 1];
-  const double adtv = fac / V.vol[i];
+  const double adtv = div_(fac, V.vol[i]);
   RkAccess ra(P, iStage);
   R rs[5];
   if (ra.rd) {
@@ -2823,7 +2830,7 @@ __global__ void __launch_bounds__(kBlock) kCellDt(View<R> V) {
         const double u1 = V.prim[n + i], v1 = V.prim[2 * n + i], w1 = V.prim[3 * n + i];
         if (const double *Q = symmetryQ(V, code)) {
           // an interior face to the cell's reflection (momentum reflected)
-          const double ir1 = 1.0 / V.cv[i];
+          const double ir1 = div_(1.0, V.cv[i]);
           const double m1[3] = {V.cv[n + i], V.cv[2 * n + i], V.cv[3 * n + i]};
           double m2[3];
           reflect3(Q, m1, m2);
@@ -2838,7 +2845,7 @@ __global__ void __launch_bounds__(kBlock) kCellDt(View<R> V) {
         sum = sum + (fabs(vc - 0.0) + V.dv[2 * n + i]) * nm;
       }
     }
-    dt = V.vol[i] / sum;
+    dt = div_(V.vol[i], sum);
   }
   blockMinDt(V.sc, dt);
 }
@@ -2973,7 +2980,9 @@ struct Launch {
     if constexpr (!Layout<R>::packed) {
       if (V.p.reconst == 2) {
         const int b = shapeFor(V, 5LL * V.nc).block;
-        kWenoVar<R><<<dim3((V.nc + b - 1) / b, 5), b, 0, s>>>(V, V.gradRaw);
+        const dim3 grid((V.nc + b - 1) / b, 5);
+        if (V.wenoW) kWenoVar<R, true><<<grid, b, 0, s>>>(V, V.gradRaw);
+        else kWenoVar<R, false><<<grid, b, 0, s>>>(V, V.gradRaw);
         return;
       }
     }

@@ -9,8 +9,6 @@
 
 namespace rflu {
 
-__host__ __device__ inline double sqrt_(double x) { return sqrt(x); }
-__host__ __device__ inline float sqrt_(float x) { return sqrtf(x); }
 __host__ __device__ inline double fabs_(double x) { return fabs(x); }
 __host__ __device__ inline float fabs_(float x) { return fabsf(x); }
 __host__ __device__ inline double copysign_(double a, double b) { return copysign(a, b); }
@@ -20,12 +18,12 @@ __host__ __device__ inline float copysign_(float a, float b) { return copysignf(
 __host__ __device__ inline double powConstExp(double x, double y) { return pow(x, y); }
 __host__ __device__ inline float powConstExp(float x, float y) { return powf(x, y); }
 // Fortran MIN/MAX of two reals (first argument kept on ties)
-template <typename S> __host__ __device__ inline S fmin2(const S &a, const S &b) { return (b < a) ? b : a; }
-template <typename S> __host__ __device__ inline S fmax2(const S &a, const S &b) { return (b > a) ? b : a; }
+template <typename S> __host__ __device__ inline S fmin2(const S &a, const S &b) { return less_(b, a) ? b : a; }
+template <typename S> __host__ __device__ inline S fmax2(const S &a, const S &b) { return less_(a, b) ? b : a; }
 
 // libfloflu/MixtPerf_*.F90
 template <typename S> __host__ __device__ inline S perfEo(S d, S g, S p, S u, S v, S w) {  // MixtPerf_E.F90:79
-  return p / (d * (g - S(1))) + S(0.5) * (u * u + v * v + w * w);
+  return div_(p, d * (g - S(1))) + S(0.5) * (u * u + v * v + w * w);
 }
 template <typename S> __host__ __device__ inline S perfHo(S cp, S t, S u, S v, S w) {      // MixtPerf_H.F90:78
   return cp * t + S(0.5) * (u * u + v * v + w * w);
@@ -36,8 +34,8 @@ template <typename S> __host__ __device__ inline S perfCGHoVm2(S g, S ho, S vm2)
 
 // modflu/RFLU_ModEntropyFixes.F90:95-106
 template <typename S> __host__ __device__ inline S entropyFixHH(S l, S d) {
-  if (l > d) return l;
-  return (l * l + d * d) / (S(2) * d);
+  if (less_(d, l)) return l;
+  return div_(l * l + d * d, S(2) * d);
 }
 
 // Roe flux with the Harten-Hyman fix, flxConv - flxDiss:
@@ -50,7 +48,7 @@ __host__ __device__ inline void roeFlux(S g, S epsentr, S dissFact, S nx, S ny, 
   S ql = ul * nx + vl * ny + wl * nz - fs;
   S qr = ur * nx + vr * ny + wr * nz - fs;
   S rh = sqrt_(rl * rr);
-  S wt = rl / (rl + rh);
+  S wt = div_(rl, rl + rh);
   S uh = wt * ul + (S(1) - wt) * ur;
   S vh = wt * vl + (S(1) - wt) * vr;
   S wh = wt * wl + (S(1) - wt) * wr;
@@ -65,9 +63,9 @@ __host__ __device__ inline void roeFlux(S g, S epsentr, S dissFact, S nx, S ny, 
   l5 = entropyFixHH(l5, efc);
   S dr = rr - rl, du = ur - ul, de = vr - vl, dw = wr - wl, dp = pr - pl;
   S dq = du * nx + de * ny + dw * nz;
-  S dv1 = (dp - rh * ah * dq) / (S(2) * ah * ah);
-  S dv5 = (dp + rh * ah * dq) / (S(2) * ah * ah);
-  S dv2 = dr - dp / (ah * ah);
+  S dv1 = div_(dp - rh * ah * dq, S(2) * ah * ah);
+  S dv5 = div_(dp + rh * ah * dq, S(2) * ah * ah);
+  S dv2 = dr - div_(dp, ah * ah);
   S t1 = l1 * dv1, t2 = l2 * dv2, t3 = l2 * rh, t5 = l5 * dv5;
   S h = S(0.5), hd = S(0.5) * dissFact;
   S fc1 = h * (ql * rl + qr * rr) * nm;
@@ -91,8 +89,8 @@ __host__ __device__ inline void hllcFlux(S g, S nx, S ny, S nz, S nm, S rl, S ul
   const S fs = S(0);
   S ql = ul * nx + vl * ny + wl * nz - fs;
   S qr = ur * nx + vr * ny + wr * nz - fs;
-  S wt1 = sqrt_(rr / rl);
-  S wt2 = S(1) / (S(1) + wt1);
+  S wt1 = sqrt_(div_(rr, rl));
+  S wt2 = div_(S(1), S(1) + wt1);
   S us = wt2 * (ul + wt1 * ur);
   S vs = wt2 * (vl + wt1 * vr);
   S ws = wt2 * (wl + wt1 * wr);
@@ -102,31 +100,31 @@ __host__ __device__ inline void hllcFlux(S g, S nx, S ny, S nz, S nm, S rl, S ul
   S as = perfCGHoVm2(g, Hs, Vms);
   S sl = fmin2(ql - al, qs - as);
   S sr = fmax2(qr + ar, qs + as);
-  if (sl > S(0)) {
+  if (pos_(sl)) {
     flx[0] = ql * rl * nm;
     flx[1] = (ql * rl * ul + pl * nx) * nm;
     flx[2] = (ql * rl * vl + pl * ny) * nm;
     flx[3] = (ql * rl * wl + pl * nz) * nm;
     flx[4] = (ql * (rl * el + pl) + pl * fs) * nm;
-  } else if (sr < S(0)) {
+  } else if (neg_(sr)) {
     flx[0] = qr * rr * nm;
     flx[1] = (qr * rr * ur + pr * nx) * nm;
     flx[2] = (qr * rr * vr + pr * ny) * nm;
     flx[3] = (qr * rr * wr + pr * nz) * nm;
     flx[4] = (qr * (rr * er + pr) + pr * fs) * nm;
   } else {
-    S sm = (rr * qr * (sr - qr) - rl * ql * (sl - ql) - pr + pl) / (rr * (sr - qr) - rl * (sl - ql));
+    S sm = div_(rr * qr * (sr - qr) - rl * ql * (sl - ql) - pr + pl, rr * (sr - qr) - rl * (sl - ql));
     S ps = pl + rl * (ql - sl) * (ql - sm);
     S rs, rus, rvs, rws, res;
-    if (sm > S(0)) {
-      S term = S(1) / (sl - sm);
+    if (pos_(sm)) {
+      S term = div_(S(1), sl - sm);
       rs = term * (sl - ql) * rl;
       rus = term * ((sl - ql) * rl * ul + (ps - pl) * nx);
       rvs = term * ((sl - ql) * rl * vl + (ps - pl) * ny);
       rws = term * ((sl - ql) * rl * wl + (ps - pl) * nz);
       res = term * ((sl - ql) * rl * el + (ps * sm - pl * ql));
     } else {
-      S term = S(1) / (sr - sm);
+      S term = div_(S(1), sr - sm);
       rs = term * (sr - qr) * rr;
       rus = term * ((sr - qr) * rr * ur + (ps - pr) * nx);
       rvs = term * ((sr - qr) * rr * vr + (ps - pr) * ny);
@@ -149,22 +147,22 @@ __host__ __device__ inline void ausmFlux(S nx, S ny, S nz, S nm, S rl, S ul, S v
   S ql = ul * nx + vl * ny + wl * nz - fs;
   S qr = ur * nx + vr * ny + wr * nz - fs;
   S af = S(0.5) * (al + ar);
-  S ml = ql / af, mla = fabs_(ml);
-  S mr = qr / af, mra = fabs_(mr);
+  S ml = div_(ql, af), mla = fabs_(ml);
+  S mr = div_(qr, af), mra = fabs_(mr);
   S mlp, wtl, mrm, wtr;
-  if (mla <= one) {
+  if (lessEq_(mla, one)) {
     mlp = S(0.25) * (ml + one) * (ml + one) + S(0.125) * (ml * ml - one) * (ml * ml - one);
     wtl = S(0.25) * (ml + one) * (ml + one) * (S(2) - ml) + S(0.1875) * ml * (ml * ml - one) * (ml * ml - one);
   } else {
     mlp = S(0.5) * (ml + mla);
-    wtl = S(0.5) * (one + ml / mla);
+    wtl = S(0.5) * (one + div_(ml, mla));
   }
-  if (mra <= one) {
+  if (lessEq_(mra, one)) {
     mrm = -S(0.25) * (mr - one) * (mr - one) - S(0.125) * (mr * mr - one) * (mr * mr - one);
     wtr = S(0.25) * (mr - one) * (mr - one) * (S(2) + mr) - S(0.1875) * mr * (mr * mr - one) * (mr * mr - one);
   } else {
     mrm = S(0.5) * (mr - mra);
-    wtr = S(0.5) * (one - mr / mra);
+    wtr = S(0.5) * (one - div_(mr, mra));
   }
   S mf = mlp + mrm, mfa = fabs_(mf);
   S mfp = S(0.5) * (mf + mfa), mfm = S(0.5) * (mf - mfa);
@@ -181,15 +179,15 @@ template <typename S>
 __host__ __device__ inline void bcondOutflowPerf(int bcOpt, S pout, S sxn, S syn, S szn, S cpgas, S mol, S rho, S rhou,
                                                  S rhov, S rhow, S rhoe, S press, S &rhob, S &rhoub, S &rhovb,
                                                  S &rhowb, S &rhoeb) {
-  S rgas = S(8314.3) / mol;
-  S gamma = cpgas / (cpgas - rgas);
-  S u = rhou / rho, v = rhov / rho, w = rhow / rho;
-  S csound = sqrt_(gamma * press / rho);
-  S mach = sqrt_(u * u + v * v + w * w) / csound;
+  S rgas = div_(S(8314.3), mol);
+  S gamma = div_(cpgas, cpgas - rgas);
+  S u = div_(rhou, rho), v = div_(rhov, rho), w = div_(rhow, rho);
+  S csound = sqrt_(div_(gamma * press, rho));
+  S mach = div_(sqrt_(u * u + v * v + w * w), csound);
   if (mach < S(1) && (bcOpt == 1 || bcOpt == 2)) {
-    S rrhoc = S(1) / (rho * csound);
+    S rrhoc = div_(S(1), rho * csound);
     S deltp = press - pout;
-    rhob = rho - deltp / (csound * csound);
+    rhob = rho - div_(deltp, csound * csound);
     S ub = u + sxn * deltp * rrhoc;
     S vb = v + syn * deltp * rrhoc;
     S wb = w + szn * deltp * rrhoc;
@@ -216,8 +214,8 @@ template <typename S>
 __host__ __device__ inline void centralPatchFlux(S nx, S ny, S nz, S nm, S rl, S rul, S rvl, S rwl, S rel, S pl, S rr,
                                                  S rur, S rvr, S rwr, S rer, S pr, S *flx) {
   const S fs = S(0);
-  S ql = (rul * nx + rvl * ny + rwl * nz) / rl - fs;
-  S qr = (rur * nx + rvr * ny + rwr * nz) / rr - fs;
+  S ql = div_(rul * nx + rvl * ny + rwl * nz, rl) - fs;
+  S qr = div_(rur * nx + rvr * ny + rwr * nz, rr) - fs;
   S h = S(0.5);
   flx[0] = h * (ql * rl + qr * rr) * nm;
   flx[1] = h * (ql * rul + pl * nx + qr * rur + pr * nx) * nm;
@@ -245,27 +243,27 @@ __host__ __device__ inline void outflowPatchFlux(int bcOpt, S pOut, S cp, S mol,
 template <typename S>
 __host__ __device__ inline void farfieldRindPerf(const double *K, S g, S nx, S ny, S nz, S rl, S rul, S rvl, S rwl,
                                                  S rel, S &rr, S &rur, S &rvr, S &rwr, S &rer, S &pr) {
-  S ul = rul / rl, vl = rvl / rl, wl = rwl / rl;
+  S ul = div_(rul, rl), vl = div_(rvl, rl), wl = div_(rwl, rl);
   S ql = ul * nx + vl * ny + wl * nz;
-  S el = rel / rl;
+  S el = div_(rel, rl);
   S sl2 = ul * ul + vl * vl + wl * wl;
   S pl = (g - S(1)) * rl * (el - S(0.5) * sl2);  // MixtPerf_P_DEoGVm2
   const S ri = S(K[1]), pi = S(K[2]), ui = S(K[4]), vi = S(K[5]), wi = S(K[6]);
   if (K[0] < 1.0) {
-    S al = sqrt_(g * pl / rl);  // MixtPerf_C_DGP
+    S al = sqrt_(div_(g * pl, rl));  // MixtPerf_C_DGP
     S pb, rb, ub, vb, wb;
     if (ql < S(0)) {
       pb = S(0.5) * (pi + pl - rl * al * ((ui - ul) * nx + (vi - vl) * ny + (wi - wl) * nz));
-      rb = ri - (pi - pb) / (al * al);
-      ub = ui - nx * (pi - pb) / (rl * al);
-      vb = vi - ny * (pi - pb) / (rl * al);
-      wb = wi - nz * (pi - pb) / (rl * al);
+      rb = ri - div_(pi - pb, al * al);
+      ub = ui - div_(nx * (pi - pb), rl * al);
+      vb = vi - div_(ny * (pi - pb), rl * al);
+      wb = wi - div_(nz * (pi - pb), rl * al);
     } else {
       pb = pi;
-      rb = rl - (pl - pi) / (al * al);
-      ub = ul + nx * (pl - pi) / (rl * al);
-      vb = vl + ny * (pl - pi) / (rl * al);
-      wb = wl + nz * (pl - pi) / (rl * al);
+      rb = rl - div_(pl - pi, al * al);
+      ub = ul + div_(nx * (pl - pi), rl * al);
+      vb = vl + div_(ny * (pl - pi), rl * al);
+      wb = wl + div_(nz * (pl - pi), rl * al);
     }
     rr = rb;
     rur = rb * ub;
@@ -297,16 +295,16 @@ __host__ __device__ inline void inflowTotAngPerf(int bcOpt, const double *K, S g
   if (bcOpt == 1 || bcOpt == 2) {  // BCOPT_SUBSONIC, BCOPT_MIXED
     const S ptot = S(K[0]), ttot = S(K[1]);
     S gm1 = g - S(1);
-    S ul = rul / rl, vl = rvl / rl, wl = rwl / rl;
+    S ul = div_(rul, rl), vl = div_(rvl, rl), wl = div_(rwl, rl);
     S a02 = g * rgas * ttot;                                           // MixtPerf_C2_GRT
     S al = sqrt_(a02 - S(0.5) * (g - S(1)) * (ul * ul + vl * vl + wl * wl));  // MixtPerf_C_Co2GUVW
     S ql = ul * nx + vl * ny + wl * nz;
     if (fabs_(ql) < al) {
       S sl = sqrt_(ul * ul + vl * vl + wl * wl);
       S eta = S(-1);
-      if (K[6] == 0.0 && sl > S(1.0e-6)) eta = ql / sl;  // BCOPT_FIXED_NO, a well-defined angle
+      if (K[6] == 0.0 && sl > S(1.0e-6)) eta = div_(ql, sl);  // BCOPT_FIXED_NO, a well-defined angle
       S Rm = al - S(0.5) * gm1 * ql;
-      S disc = S(0.5) * gm1 * (eta * eta) * (a02 / (Rm * Rm) * (S(1) + S(0.5) * gm1 * (eta * eta)) - S(1));
+      S disc = S(0.5) * gm1 * (eta * eta) * (div_(a02, Rm * Rm) * (S(1) + S(0.5) * gm1 * (eta * eta)) - S(1));
       S ar, tr, sr;
       if (disc < S(0)) {
         ar = sqrt_(a02);
@@ -314,17 +312,17 @@ __host__ __device__ inline void inflowTotAngPerf(int bcOpt, const double *K, S g
         pr = ptot;
         sr = S(0);
       } else {
-        ar = Rm / (S(1) + S(0.5) * gm1 * eta * eta) * (S(1) + sqrt_(disc));
-        tr = ar * ar / (g * rgas);                              // MixtPerf_T_CGR
-        pr = ptot * powConstExp(tr / ttot, g / (g - S(1)));     // MixtPerf_P_GPoTTo
+        ar = div_(Rm, S(1) + S(0.5) * gm1 * eta * eta) * (S(1) + sqrt_(disc));
+        tr = div_(ar * ar, g * rgas);                              // MixtPerf_T_CGR
+        pr = ptot * powConstExp(div_(tr, ttot), div_(g, g - S(1)));     // MixtPerf_P_GPoTTo
         S c2 = ar * ar;                                          // MixtPerf_Vm_C2Co2G
-        sr = (a02 > c2) ? sqrt_(S(2) / (g - S(1)) * (a02 - c2)) : S(0);
+        sr = (a02 > c2) ? sqrt_(div_(S(2), g - S(1)) * (a02 - c2)) : S(0);
       }
-      rr = pr / (rgas * tr);  // MixtPerf_D_PRT
+      rr = div_(pr, rgas * tr);  // MixtPerf_D_PRT
       S ur = sr * S(K[2]) * S(K[4]);
       S vr = sr * S(K[3]);
       S wr = sr * S(K[2]) * S(K[5]);
-      rer = rr * (pr / (rr * (g - S(1))) + S(0.5) * sr * sr);  // MixtPerf_Eo_DGPVm
+      rer = rr * (div_(pr, rr * (g - S(1))) + S(0.5) * sr * sr);  // MixtPerf_Eo_DGPVm
       rur = rr * ur;
       rvr = rr * vr;
       rwr = rr * wr;
@@ -363,16 +361,16 @@ __host__ __device__ inline void inflowVelTempPerf(int bcOpt, const double *K, S 
 template <typename S>
 __host__ __device__ inline S slipWallRindPerf(S g, S nx, S ny, S nz, S rl, S rul, S rvl, S rwl, S pl) {
   const S fs = S(0);
-  S irl = S(1) / rl;
+  S irl = div_(S(1), rl);
   S ul = irl * rul, vl = irl * rvl, wl = irl * rwl;
   S ql = ul * nx + vl * ny + wl * nz - fs;
-  S al = sqrt_(g * pl / rl);
+  S al = sqrt_(div_(g * pl, rl));
   if (ql < S(0)) {
-    S term = S(1) + S(0.5) * (g - S(1)) * ql / al;
-    return pl * powConstExp(term, S(2) * g / (g - S(1)));
+    S term = S(1) + div_(S(0.5) * (g - S(1)) * ql, al);
+    return pl * powConstExp(term, div_(S(2) * g, g - S(1)));
   }
-  S term = (g + S(1)) / S(4);
-  return pl + term * rl * ql * (ql + sqrt_(al * al + term * term * ql * ql) / term);
+  S term = div_(g + S(1), S(4));
+  return pl + term * rl * ql * (ql + div_(sqrt_(al * al + term * term * ql * ql), term));
 }
 
 // Injection patch flux (RFLU_CentralFirstPatch.F90:1043-1127,
@@ -386,8 +384,8 @@ __host__ __device__ inline void injectionPatchFlux(const double *K, S g, S cp, S
   const S fs = S(0);
   if (K[0] > 0.0) {
     const S minj = S(K[0]), tinj = S(K[1]);
-    S rb = pl / (rgas * tinj);  // MixtPerf_D_PRT
-    S qb = -minj / rb + fs;
+    S rb = div_(pl, rgas * tinj);  // MixtPerf_D_PRT
+    S qb = div_(-minj, rb) + fs;
     S ub = qb * nx, vb = qb * ny, wb = qb * nz;
     S hb = perfHo(cp, tinj, ub, vb, wb);
     flx[0] = -minj * nm;
@@ -424,18 +422,18 @@ __host__ __device__ inline void symmetricEigen3(const S m[9], S vec[9], S val[3]
   const S tol = S(1.0e-24);
   for (int sweep = 0; sweep < 50; ++sweep) {
     S off = r[3] * r[3] + r[6] * r[6] + r[7] * r[7];
-    if (off <= tol * total) break;
+    if (lessEq_(off, tol * total)) break;
 #pragma unroll
     for (int ip = 0; ip < 2; ++ip)
 #pragma unroll
       for (int iq = ip + 1; iq < 3; ++iq) {
         const int pq = ip + 3 * iq, pp = ip + 3 * ip, qq = iq + 3 * iq;
-        if (r[pq] != S(0)) {
-          S theta = (r[qq] - r[pp]) / (S(2) * r[pq]);
+        if (nonZero_(r[pq])) {
+          S theta = div_(r[qq] - r[pp], S(2) * r[pq]);
           S t;
-          if (fabs_(theta) > S(1.0e150)) t = S(0.5) / theta;
-          else t = copysign_(S(1), theta) / (fabs_(theta) + sqrt_(theta * theta + S(1)));
-          S c = S(1) / sqrt_(t * t + S(1));
+          if (less_(S(1.0e150), fabs_(theta))) t = div_(S(0.5), theta);
+          else t = div_(copysign_(S(1), theta), fabs_(theta) + sqrt_(theta * theta + S(1)));
+          S c = div_(S(1), sqrt_(t * t + S(1)));
           S s = t * c;
           const int ir = 3 - ip - iq;
           S arp = r[ir + 3 * ip], arq = r[ir + 3 * iq];
@@ -464,11 +462,11 @@ __host__ __device__ inline void symmetricEigen3(const S m[9], S vec[9], S val[3]
 #pragma unroll
     for (int k = 0; k < 3; ++k) { S x = vec[k + 3 * a]; vec[k + 3 * a] = vec[k + 3 * b]; vec[k + 3 * b] = x; }
   };
-  const bool m1 = val[1] < val[0];
-  const bool m2 = val[2] < (m1 ? val[1] : val[0]);
+  const bool m1 = less_(val[1], val[0]);
+  const bool m2 = less_(val[2], m1 ? val[1] : val[0]);
   if (m2) swapCols(0, 2);
   else if (m1) swapCols(0, 1);
-  if (val[2] < val[1]) swapCols(1, 2);
+  if (less_(val[2], val[1])) swapCols(1, 2);
 }
 
 // Whether eigenvalues j < k (ascending) lie in one group of the eigen-frame
@@ -564,7 +562,7 @@ __host__ __device__ inline void symmetricEigen3(const Dual<N, T> m[9], Dual<N, T
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         if (k == j || l[j] == l[k] || mergedPair(l, j < k ? j : k, j < k ? k : j)) continue;
-        const T coef = (a[3 * k] * sa[0] + a[3 * k + 1] * sa[1] + a[3 * k + 2] * sa[2]) / (l[j] - l[k]);
+        const T coef = div_(a[3 * k] * sa[0] + a[3 * k + 1] * sa[1] + a[3 * k + 2] * sa[2], l[j] - l[k]);
 #pragma unroll
         for (int r = 0; r < 3; ++r) vec[r + 3 * j].d[q] += coef * a[r + 3 * k];
       }

@@ -11,10 +11,12 @@
 #pragma once
 #include <cmath>
 
+#include "dual.cuh"
+
 namespace rflu {
 
 template <typename T>
-__host__ __device__ inline T sgn1(T x) { return (x < T(0)) ? T(-1) : T(1); }
+__host__ __device__ inline T sgn1(T x) { return neg_(x) ? T(-1) : T(1); }
 
 // T: double in the FP64 modes, float in the mixed mode (the arithmetic of
 // each mode's flux); the numerics parameters arrive in double.
@@ -25,31 +27,31 @@ __host__ __device__ inline void roe2Adjoint(double gD, double cpD, double epsD, 
   // ---------------- forward ----------------
   const T rl = L[0], ul = L[1], vl = L[2], wl = L[3], pl = L[4];
   const T rr = R[0], ur = R[1], vr = R[2], wr = R[3], pr = R[4];
-  const T gc = cp - cp / g;
-  const T tl = pl / (rl * gc), tr = pr / (rr * gc);
+  const T gc = cp - div_(cp, g);
+  const T tl = div_(pl, rl * gc), tr = div_(pr, rr * gc);
   const T Hl = cp * tl + T(0.5) * (ul * ul + vl * vl + wl * wl);
   const T Hr = cp * tr + T(0.5) * (ur * ur + vr * vr + wr * wr);
   const T ql = ul * nx + vl * ny + wl * nz;
   const T qr = ur * nx + vr * ny + wr * nz;
-  const T rh = sqrt(rl * rr);
-  const T wt = rl / (rl + rh), w1 = T(1.0) - wt;
+  const T rh = sqrt_(rl * rr);
+  const T wt = div_(rl, rl + rh), w1 = T(1.0) - wt;
   const T uh = wt * ul + w1 * ur, vh = wt * vl + w1 * vr, wh = wt * wl + w1 * wr;
   const T Hh = wt * Hl + w1 * Hr;
   const T qh = uh * nx + vh * ny + wh * nz;
   const T sh = T(0.5) * (uh * uh + vh * vh + wh * wh);
-  const T ah = sqrt((g - T(1.0)) * (Hh - sh));
+  const T ah = sqrt_((g - T(1.0)) * (Hh - sh));
   const T L1 = fabs(qh - ah), L2 = fabs(qh), L5 = fabs(qh + ah);
   const T efc = eps * L5;
-  const bool k1 = L1 > efc, k2 = L2 > efc, k5 = L5 > efc;
-  const T l1 = k1 ? L1 : (L1 * L1 + efc * efc) / (T(2.0) * efc);
-  const T l2 = k2 ? L2 : (L2 * L2 + efc * efc) / (T(2.0) * efc);
-  const T l5 = k5 ? L5 : (L5 * L5 + efc * efc) / (T(2.0) * efc);
+  const bool k1 = less_(efc, L1), k2 = less_(efc, L2), k5 = less_(efc, L5);
+  const T l1 = k1 ? L1 : div_(L1 * L1 + efc * efc, T(2.0) * efc);
+  const T l2 = k2 ? L2 : div_(L2 * L2 + efc * efc, T(2.0) * efc);
+  const T l5 = k5 ? L5 : div_(L5 * L5 + efc * efc, T(2.0) * efc);
   const T dr = rr - rl, du = ur - ul, de = vr - vl, dw = wr - wl, dp = pr - pl;
   const T dq = du * nx + de * ny + dw * nz;
   const T den = T(2.0) * ah * ah;
-  const T dv1 = (dp - rh * ah * dq) / den;
-  const T dv5 = (dp + rh * ah * dq) / den;
-  const T dv2 = dr - dp / (ah * ah);
+  const T dv1 = div_(dp - rh * ah * dq, den);
+  const T dv5 = div_(dp + rh * ah * dq, den);
+  const T dv2 = dr - div_(dp, ah * ah);
   const T t1 = l1 * dv1, t2 = l2 * dv2, t3 = l2 * rh, t5 = l5 * dv5;
 
   // ---------------- reverse ----------------
@@ -96,26 +98,26 @@ __host__ __device__ inline void roe2Adjoint(double gD, double cpD, double epsD, 
   T dv1b = t1b * l1, dv2b = t2b * l2, dv5b = t5b * l5;
   T rhb = t3b * l2;
   // dv1, dv5, dv2
-  T dpb = (dv1b + dv5b) / den - dv2b / (ah * ah);
-  rhb += (-dv1b + dv5b) * ah * dq / den;
-  ahb += dv1b * (-rh * dq / den - T(2.0) * dv1 / ah) + dv5b * (rh * dq / den - T(2.0) * dv5 / ah) +
-         dv2b * (T(2.0) * dp / (ah * ah * ah));
-  dqb += (-dv1b + dv5b) * rh * ah / den;
+  T dpb = div_(dv1b + dv5b, den) - div_(dv2b, ah * ah);
+  rhb += div_((-dv1b + dv5b) * ah * dq, den);
+  ahb += dv1b * (div_(-rh * dq, den) - div_(T(2.0) * dv1, ah)) + dv5b * (div_(rh * dq, den) - div_(T(2.0) * dv5, ah)) +
+         dv2b * div_(T(2.0) * dp, ah * ah * ah);
+  dqb += div_((-dv1b + dv5b) * rh * ah, den);
   T drb = dv2b;
   dub += dqb * nx;
   deb += dqb * ny;
   dwb += dqb * nz;
   // entropy fix
   T L1b = 0, L2b = 0, L5b = 0, efcb = 0;
-  if (k1) L1b += l1b; else { L1b += l1b * L1 / efc; efcb += l1b * (efc * efc - L1 * L1) / (T(2.0) * efc * efc); }
-  if (k2) L2b += l2b; else { L2b += l2b * L2 / efc; efcb += l2b * (efc * efc - L2 * L2) / (T(2.0) * efc * efc); }
-  if (k5) L5b += l5b; else { L5b += l5b * L5 / efc; efcb += l5b * (efc * efc - L5 * L5) / (T(2.0) * efc * efc); }
+  if (k1) L1b += l1b; else { L1b += div_(l1b * L1, efc); efcb += div_(l1b * (efc * efc - L1 * L1), T(2.0) * efc * efc); }
+  if (k2) L2b += l2b; else { L2b += div_(l2b * L2, efc); efcb += div_(l2b * (efc * efc - L2 * L2), T(2.0) * efc * efc); }
+  if (k5) L5b += l5b; else { L5b += div_(l5b * L5, efc); efcb += div_(l5b * (efc * efc - L5 * L5), T(2.0) * efc * efc); }
   L5b += efcb * eps;
   const T s1 = sgn1(qh - ah), s2 = sgn1(qh), s5 = sgn1(qh + ah);
   qhb += L1b * s1 + L2b * s2 + L5b * s5;
   ahb += -L1b * s1 + L5b * s5;
-  // ah = sqrt((g-1)(Hh - sh))
-  const T ah2b = ahb / (T(2.0) * ah);
+  // ah = sqrt_((g-1)(Hh - sh))
+  const T ah2b = div_(ahb, T(2.0) * ah);
   Hhb += ah2b * (g - T(1.0));
   shb -= ah2b * (g - T(1.0));
   uhb += shb * uh + qhb * nx;
@@ -128,10 +130,10 @@ __host__ __device__ inline void roe2Adjoint(double gD, double cpD, double epsD, 
   wlb += whb * wt; wrb += whb * w1;
   Hlb += Hhb * wt; Hrb += Hhb * w1;
   const T s = rl + rh;
-  rlb += wtb * rh / (s * s);
-  rhb += -wtb * rl / (s * s);
-  rlb += rhb * rr / (T(2.0) * rh);
-  rrb += rhb * rl / (T(2.0) * rh);
+  rlb += div_(wtb * rh, s * s);
+  rhb += div_(-wtb * rl, s * s);
+  rlb += div_(rhb * rr, T(2.0) * rh);
+  rrb += div_(rhb * rl, T(2.0) * rh);
   // differences
   rrb += drb; rlb -= drb;
   urb += dub; ulb -= dub;
@@ -142,11 +144,11 @@ __host__ __device__ inline void roe2Adjoint(double gD, double cpD, double epsD, 
   ulb += qlb * nx; vlb += qlb * ny; wlb += qlb * nz;
   urb += qrb * nx; vrb += qrb * ny; wrb += qrb * nz;
   // total enthalpies: H = cp p/(rho gc) + |u|^2/2
-  plb += Hlb * cp / (rl * gc);
-  rlb -= Hlb * cp * tl / rl;
+  plb += div_(Hlb * cp, rl * gc);
+  rlb -= div_(Hlb * cp * tl, rl);
   ulb += Hlb * ul; vlb += Hlb * vl; wlb += Hlb * wl;
-  prb += Hrb * cp / (rr * gc);
-  rrb -= Hrb * cp * tr / rr;
+  prb += div_(Hrb * cp, rr * gc);
+  rrb -= div_(Hrb * cp * tr, rr);
   urb += Hrb * ur; vrb += Hrb * vr; wrb += Hrb * wr;
   Lb[0] = rlb; Lb[1] = ulb; Lb[2] = vlb; Lb[3] = wlb; Lb[4] = plb;
   Rb[0] = rrb; Rb[1] = urb; Rb[2] = vrb; Rb[3] = wrb; Rb[4] = prb;
