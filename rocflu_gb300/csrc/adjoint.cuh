@@ -33,6 +33,7 @@
 // first-order perturbation in the tangent and the adjoint alike).
 #pragma once
 #include "dual.cuh"
+#include "hllc_adjoint.cuh"
 #include "roe_adjoint.cuh"
 
 namespace rflu {
@@ -260,13 +261,29 @@ __global__ void kTanInit(View<R> V, AdjWork<R> W, const double *cvDotRef) {
   for (int k = 0; k < 3; ++k) W.dvd[k * n + i] = (R)dv[k].d[0];
 }
 
+// haveG: W.G and W.Gbar hold the unlimited gradient and its derivative (the
+// fixed-point sums, which the adjoint's forward pass takes too, so that both
+// hold an idle eigen-frame axis at the same factor).
 template <typename R>
-__global__ void __launch_bounds__(kBlock) kTanGrad(View<R> V, AdjWork<R> W) {
+__global__ void __launch_bounds__(kBlock) kTanGrad(View<R> V, AdjWork<R> W, bool haveG) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   Dual<1, R> g[15];
-  gradLimitCell(V, TanLoad<R>{V, W}, i, g);
   const size_t n = V.nc;
+  const TanLoad<R> td{V, W};
+  if (haveG) {
+    Dual<1, R> q[5];
+    td.prim5(i, q);
+#pragma unroll
+    for (int k = 0; k < 15; ++k) {
+      g[k].v = W.G[k * n + i];
+      g[k].d[0] = W.Gbar[k * n + i];
+    }
+    if (V.cSlot && V.cSlot[i] >= 0) constrainedGrad(V, td, i, V.cSlot[i], q, g);
+    limitCell(V, td, i, q, g);
+  } else {
+    gradLimitCell(V, td, i, g);
+  }
   if (isWeno(V.p)) {
     // the unsmoothed gradient and its derivative, for kTanWeno
 #pragma unroll
@@ -283,6 +300,90 @@ __global__ void __launch_bounds__(kBlock) kTanGrad(View<R> V, AdjWork<R> W) {
     W.gradd[k * n + i] = g[k].d[0];
   }
   storeGrad(V, i, gv);
+}
+
+// Venkatakrishnan factor (RFLU_ModLimiters.F90:494-516) of one face side.
+template <typename S>
+__device__ inline S venkat(S dext, S d2, S epsq) {
+  S numer = (dext * dext + epsq) * d2 + S(2) * d2 * d2 * dext;
+  S denom = d2 * (dext * dext + S(2) * d2 * d2 + dext * d2 + epsq);
+  return div_(numer, denom + S(1.0e-12));
+}
+
+// The tangent of the componentwise limiters (and of none) along the branch
+// kAdjGradFwd recorded: with the unlimited gradient G (W.G), its derivative
+// along the direction (W.Gbar; the fit is linear, so the same sums of the
+// direction's primitive state) and the factor l = phi(dext, d2) of the active
+// face and neighbour, the limited gradient's derivative is l dG + dl G.  Two
+// passes of the sums on the integer pipe and one of the limiter take the place
+// of the sums and every face's factor on dual numbers (kTanGrad; 196,608
+// tetrahedra: tangent and adjoint
+// 4.43 -> 3.00 ms with the adjoint's own term).  Constrained cells' rows carry their constraint values'
+// derivatives and run on dual numbers here.
+template <typename R>
+__global__ void __launch_bounds__(kBlock) kTanLimit(View<R> V, AdjWork<R> W) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= V.nc) return;
+  const size_t n = V.nc;
+  const PlainLoad<R> ld{V};
+  R gd[15];
+#pragma unroll
+  for (int k = 0; k < 15; ++k) gd[k] = W.Gbar[k * n + i];
+  if (V.cSlot && V.cSlot[i] >= 0) {
+    const TanLoad<R> td{V, W};
+    Dual<1, R> q[5], g[15];
+    td.prim5(i, q);
+#pragma unroll
+    for (int k = 0; k < 15; ++k) {
+      g[k].v = W.G[k * n + i];
+      g[k].d[0] = gd[k];
+    }
+    constrainedGrad(V, td, i, V.cSlot[i], q, g);
+#pragma unroll
+    for (int k = 0; k < 15; ++k) gd[k] = g[k].d[0];
+  }
+  const int rc = V.p.reconst;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const R G[3] = {W.G[(3 * k) * n + i], W.G[(3 * k + 1) * n + i], W.G[(3 * k + 2) * n + i]};
+    const R l = W.lim[k * n + i];
+    const int es = W.estar[k * n + i];
+    R ldot = R(0);
+    if (es >= 0) {
+      R d[3];
+      limiterFaceOffset(V, V.cfEnt[es], d);
+      const R d2 = -(G[0] * d[0] + G[1] * d[1] + G[2] * d[2]);
+      const R d2dot = -(gd[3 * k] * d[0] + gd[3 * k + 1] * d[1] + gd[3 * k + 2] * d[2]);
+      const int js = W.jstar[k * n + i];
+      const R qi = ld.prim(k, i), qid = W.primd[k * n + i];
+      R ext = qi, extd = qid;
+      if (js >= 0) {
+        ext = ld.prim(k, js);
+        extd = W.primd[k * n + js];
+      } else if (js <= kMirrorNb && k >= 1 && k <= 3) {  // the cell's reflection across a symmetry face
+        const double *Q = V.patchK + kPatchK * V.bpatch[kMirrorNb - js];
+        const R u[3] = {ld.prim(1, i), ld.prim(2, i), ld.prim(3, i)};
+        const R ud[3] = {W.primd[n + i], W.primd[2 * n + i], W.primd[3 * n + i]};
+        R m[3], md[3];
+        reflect3(Q, u, m);
+        reflect3(Q, ud, md);
+        ext = k == 1 ? m[0] : k == 2 ? m[1] : m[2];
+        extd = k == 1 ? md[0] : k == 2 ? md[1] : md[2];
+      }
+      const R dext = ext - qi, dextd = extd - qid;
+      if (rc == 11) {
+        using D1 = Dual<1, R>;
+        D1 a(dext), b(d2);
+        a.d[0] = dextd;
+        b.d[0] = d2dot;
+        ldot = venkat(a, b, D1(V.epsq[i])).d[0];
+      } else {
+        ldot = div_(dextd - div_(dext, d2) * d2dot, d2);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) W.gradd[(3 * k + c) * n + i] = l * gd[3 * k + c] + ldot * G[c];
+  }
 }
 
 // The simple limiter after the WENO smoothing (RFLU_LimitGradCellsSimple,
@@ -387,14 +488,6 @@ __global__ void kAdjLambda(View<R> V, AdjWork<R> W, const double *lamRef) {
   const int o = V.refId[i];
 #pragma unroll
   for (int k = 0; k < 5; ++k) W.cvd[(size_t)k * V.nc + i] = (R)lamRef[5 * (size_t)o + k];
-}
-
-// Venkatakrishnan factor (RFLU_ModLimiters.F90:494-516) of one face side.
-template <typename S>
-__device__ inline S venkat(S dext, S d2, S epsq) {
-  S numer = (dext * dext + epsq) * d2 + S(2) * d2 * d2 * dext;
-  S denom = d2 * (dext * dext + S(2) * d2 * d2 + dext * d2 + epsq);
-  return div_(numer, denom + S(1.0e-12));
 }
 
 // The eigen-frame velocity limiter of one cell (RECONST 10,
@@ -685,8 +778,9 @@ __device__ inline void velFrameReverse(const View<R> &V, const L &ld, int i, con
 // with lamRef, also kAdjLambda's copy of the cell's adjoint seed.
 // kVel: compiled with the eigen-frame velocity limiter (RECONST 10), so that
 // the other limiters keep their smaller register allocation.
+// haveG: W.G already holds the unlimited gradient (the fixed-point sums).
 template <typename R, bool kVel>
-__global__ void __launch_bounds__(kBlock) kAdjGradFwd(View<R> V, AdjWork<R> W, const double *lamRef) {
+__global__ void __launch_bounds__(kBlock) kAdjGradFwd(View<R> V, AdjWork<R> W, const double *lamRef, bool haveG) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const size_t n = V.nc;
@@ -750,6 +844,9 @@ __global__ void __launch_bounds__(kBlock) kAdjGradFwd(View<R> V, AdjWork<R> W, c
       const int sl = V.cSlot[i];
       if (sl >= 0) constrainedGrad(V, ld, i, sl, q, g);
     }
+  } else if (haveG) {
+#pragma unroll
+    for (int k = 0; k < 15; ++k) g[k] = W.G[k * n + i];
   } else {
     for (int s = V.stOff[i]; s < V.stOff[i + 1]; ++s) {
       const int j = V.stIdx[s];
@@ -774,8 +871,10 @@ __global__ void __launch_bounds__(kBlock) kAdjGradFwd(View<R> V, AdjWork<R> W, c
       if (sl >= 0) constrainedGrad(V, ld, i, sl, q, g);
     }
   }
+  if (!haveG) {
 #pragma unroll
-  for (int k = 0; k < 15; ++k) W.G[k * n + i] = g[k];
+    for (int k = 0; k < 15; ++k) W.G[k * n + i] = g[k];
+  }
   const int rc = V.p.reconst;
   R lim[5] = {R(1), R(1), R(1), R(1), R(1)};
   int es[5] = {-1, -1, -1, -1, -1}, js[5] = {-1, -1, -1, -1, -1};
@@ -1017,11 +1116,14 @@ __device__ inline void contract(const Dual<N, T> *flx, const T *fbar, T *out) {
 }
 
 // Face adjoints of faces t0 .. t1-1 (interior faces first, then boundary
-// faces).  kRoe2 compiles only the second-order Roe interior path (its
-// hand-written reverse sweep), so that the common case is not held to the
-// register allocation of the dual-number paths; the launcher gives it the
-// interior faces of such runs and the generic kernel the rest.
-template <typename R, bool kRoe2>
+// faces).  kFlux 1 (Roe) and 3 (HLLC) compile only that flux's second-order
+// interior path, a hand-written reverse sweep, so that the common cases are
+// not held to the register allocation of the dual-number paths (255, which
+// seed six directions per side through the flux); the launcher gives them the
+// interior faces of such runs and the generic kernel (0) the rest.  Measured
+// for HLLC, mixed mode, 95,232 faces: 12 stage adjoints of an
+// unrolled gradient 2.85 -> 2.53 ms.
+template <typename R, int kFlux>
 __global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int t0, int t1) {
   const int t = t0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= t1) return;
@@ -1038,7 +1140,7 @@ __global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int 
     faceNormal(V, f, nx, ny, nz, nm);
 #pragma unroll
     for (int k = 0; k < 5; ++k) fbar[k] = W.cvd[k * n + c1] - W.cvd[k * n + c2];
-    if (!kRoe2 && P.spaceOrder == 1) {
+    if (kFlux == 0 && P.spaceOrder == 1) {
       // first order: FP64 from cv and dv in every mode (as the primal)
       using D8 = Dual<8>;
       D8 cl[5], dl[3], cr[5], dr[3], flx[5];
@@ -1067,7 +1169,11 @@ __global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int 
       faceOffset(V, f, 1, dr);
       faceState(V, ld, c1, dl[0], dl[1], dl[2], L, irl);
       faceState(V, ld, c2, dr[0], dr[1], dr[2], Rt, irr);
-      if (kRoe2 || P.spaceDiscr == 1) {
+      if constexpr (kFlux == 3) {
+        hllc2Adjoint(prm<R>(P.refGamma, P.refGammaF), nx, ny, nz, nm, L, irl, Rt, irr, fbar, out, out + 6);
+        return;
+      }
+      if (kFlux == 1 || P.spaceDiscr == 1) {
         // Roe: hand-written reverse sweep in the mode's arithmetic (no
         // dependence on the cell 1/rho)
         roe2Adjoint(P.refGamma, P.refCp, P.epsEntr, P.dissFact, nx, ny, nz, nm, L, Rt, fbar, out, out + 6);
@@ -1085,13 +1191,13 @@ __global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int 
         }
         ia = side ? D6(irl) : D6::seed(irl, 5);
         ib = side ? D6::seed(irr, 5) : D6(irr);
-        if constexpr (!kRoe2) {
+        if constexpr (kFlux == 0) {
           riemann2(P, D6(nx), D6(ny), D6(nz), D6(nm), a, ia, b, ib, flx);
           contract(flx, fbar, out + 6 * side);
         }
       }
     }
-  } else if constexpr (!kRoe2) {
+  } else if constexpr (kFlux == 0) {
     const int b = t - V.nf, c = V.bcell[b], ip = V.bpatch[b];
     const int type = V.patchType[ip], order = V.patchOrder[ip];
 #pragma unroll
@@ -1174,17 +1280,20 @@ __global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int 
 // gradient own-term.  kVel: with the eigen-frame velocity limiter (RECONST 10).
 // FP64 layouts: the own term of the LSQ gradient's transpose (or, for a
 // constrained variable, of its rows) on the cell's primitive adjoint.
+// Every member's difference subtracts the cell's value, so the term is one dot
+// product with the sum of the cell's weights (View::wSum, formed once per
+// context) instead of one per member: 15 FP64 instructions instead of 600 on
+// 40-member stencils (kAdjCell1, 196,608 tetrahedra: tangent and adjoint 4.43 -> 3.00 ms with
+// the tangent of kTanLimit and the closed form in kAdjCell2).
 template <typename R>
 __device__ inline void adjOwnTermFp64(const View<R> &V, int i, const R *gb, R *qb) {
+  const size_t n = V.nc;
   int sl;
   const int cm = constrMask(V, i, sl);
-  for (int s = V.stOff[i]; s < V.stOff[i + 1]; ++s) {
-    R wx, wy, wz;
-    lsqWeight(V, i, s, wx, wy, wz);
+  const R sx = V.wSum[i], sy = V.wSum[n + i], sz = V.wSum[2 * n + i];
 #pragma unroll
-    for (int k = 0; k < 5; ++k)
-      if (!((cm >> k) & 1)) qb[k] -= wx * gb[3 * k] + wy * gb[3 * k + 1] + wz * gb[3 * k + 2];
-  }
+  for (int k = 0; k < 5; ++k)
+    if (!((cm >> k) & 1)) qb[k] -= sx * gb[3 * k] + sy * gb[3 * k + 1] + sz * gb[3 * k + 2];
   if (cm) constrOwnTerm(V, i, sl, gb, qb);
 }
 
@@ -1771,24 +1880,32 @@ __global__ void __launch_bounds__(kBlock) kAdjCell2(View<R> V, AdjWork<R> W, dou
 #pragma unroll
     for (int m = 0; m < 5; ++m) outRef[5 * (size_t)o + m] = (double)out[m];
   } else {
-    using D5 = Dual<5>;
-    D5 cv[5], q[5], dv[3];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) cv[k] = D5::seed(V.cv[k * n + j], k);
-    primFromCv(V.p, cv, q, dv);
-    double dvb[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) dvb[k] = W.dvbar[k * n + j];
-    dvb[0] += pcon;
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      double s = W.cvbarD[m * n + j];
-#pragma unroll
-      for (int k = 0; k < 5; ++k) s += (double)qb[k] * q[k].d[m];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) s += dvb[k] * dv[k].d[m];
-      outRef[5 * (size_t)o + m] = s;
+    // the transpose of primFromCv in closed form: q = (rho, m/rho, p),
+    // dv = (p, T, c) with p = (g-1)(rho E - |m|^2/(2 rho)), T = p/(rho gc),
+    // c = sqrt(g gc T)
+    const double g = V.p.gRT, gc = V.p.gcR;
+    const double ir = div_(1.0, V.cv[j]);
+    const double u = ir * V.cv[n + j], v = ir * V.cv[2 * n + j], w = ir * V.cv[3 * n + j];
+    const double ke = 0.5 * (u * u + v * v + w * w);
+    double pb = (double)qb[4] + (W.dvbar[j] + pcon), rb = 0.0;
+    const double b1 = W.dvbar[n + j], b2 = W.dvbar[2 * n + j];
+    if (nonZero_(b1) || nonZero_(b2)) {
+      const double t = div_((g - 1.0) * (ir * V.cv[4 * n + j] - ke), gc), c = sqrt_(g * gc * t);
+      const double tb = b1 + div_(0.5 * g * gc * b2, c);
+      pb += div_(tb * ir, gc);
+      rb = -(tb * t * ir);  // dT/drho at fixed p
     }
+    const double g1 = g - 1.0, hp = g1 * pb;
+    double out[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) out[m] = W.cvbarD[m * n + j];
+    out[0] += (double)qb[0] + rb + hp * ke - ir * ((double)qb[1] * u + (double)qb[2] * v + (double)qb[3] * w);
+    out[1] += ir * (double)qb[1] - hp * u;
+    out[2] += ir * (double)qb[2] - hp * v;
+    out[3] += ir * (double)qb[3] - hp * w;
+    out[4] += hp;
+#pragma unroll
+    for (int m = 0; m < 5; ++m) outRef[5 * (size_t)o + m] = out[m];
   }
 }
 
@@ -1896,14 +2013,28 @@ struct AdjointOps {
     const size_t nT = (size_t)V.nf + V.nb;
     AdjWork<R> W = carveAdjWork<R>(work, V.nc, nT);
     kTanInit<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, cvDotRef);
-    if (V.p.spaceOrder > 1) kTanGrad<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
+    const int rc = V.p.reconst;
+    if (Launch<R>::fixedSums(V) && (rc == 0 || rc == 100 || rc == 11)) {
+      gradFwd(V, W, nullptr, s);
+      Launch<R>::launchFixed(V, W.primd, W.Gbar, false, s);
+      kTanLimit<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
+    } else if (V.p.spaceOrder > 1) {
+      const bool haveG = Launch<R>::fixedSums(V);
+      if (haveG) {
+        Launch<R>::launchFixed(V, V.prim, W.G, true, s);
+        Launch<R>::launchFixed(V, W.primd, W.Gbar, false, s);
+      }
+      kTanGrad<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, haveG);
+    }
     if (isWeno(V.p)) kTanWeno<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
     kTanFlux<R><<<RFLU_GRID(V, (long long)nT, s)>>>(V, W);
     kTanGather<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, rhsDotRef);
   }
   static void gradFwd(const View<R> &V, const AdjWork<R> &W, const double *lamRef, cudaStream_t s) {
-    if (V.p.reconst == 10) kAdjGradFwd<R, true><<<RFLU_GRID(V, V.nc, s)>>>(V, W, lamRef);
-    else kAdjGradFwd<R, false><<<RFLU_GRID(V, V.nc, s)>>>(V, W, lamRef);
+    const bool haveG = Launch<R>::fixedSums(V);
+    if (haveG) Launch<R>::launchFixed(V, V.prim, W.G, true, s);
+    if (V.p.reconst == 10) kAdjGradFwd<R, true><<<RFLU_GRID(V, V.nc, s)>>>(V, W, lamRef, haveG);
+    else kAdjGradFwd<R, false><<<RFLU_GRID(V, V.nc, s)>>>(V, W, lamRef, haveG);
     if (isWeno(V.p)) {
       if constexpr (Layout<R>::packed)
         kAdjWenoFwdLanes<R><<<RFLU_GRID(V, (long long)V.nc * adjLanes<R>(), s)>>>(V, W);
@@ -1917,6 +2048,12 @@ struct AdjointOps {
     if (isWeno(V.p)) kAdjWeno<R><<<RFLU_GRID(V, (long long)V.nc * adjLanes<R>(), s)>>>(V, W);
     kAdjCell2<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, cvBarRef);
   }
+  static void interiorFaces(const View<R> &V, const AdjWork<R> &W, cudaStream_t s) {
+    const int flux = V.p.spaceOrder > 1 ? V.p.spaceDiscr : 0;
+    if (flux == 1) kAdjFace<R, 1><<<RFLU_GRID(V, (long long)V.nf, s)>>>(V, W, 0, V.nf);
+    else if (flux == 3) kAdjFace<R, 3><<<RFLU_GRID(V, (long long)V.nf, s)>>>(V, W, 0, V.nf);
+    else kAdjFace<R, 0><<<RFLU_GRID(V, (long long)V.nf, s)>>>(V, W, 0, V.nf);
+  }
   // The boundary faces' kernel (dual numbers through the patch fluxes; few
   // faces, a small grid) runs on a second stream beside the interior faces'
   // (they write disjoint face-adjoint entries), forked from and joined
@@ -1924,19 +2061,17 @@ struct AdjointOps {
   // last wave leaves idle.
   static void faceAdjoint(const View<R> &V, const AdjWork<R> &W, cudaStream_t s) {
     const int nT = V.nf + V.nb;
-    const bool roe2 = V.p.spaceOrder > 1 && V.p.spaceDiscr == 1;
     if (V.nf == 0 || V.nb == 0) {
-      if (nT > 0 && !(roe2 && V.nb == 0)) kAdjFace<R, false><<<RFLU_GRID(V, (long long)nT, s)>>>(V, W, 0, nT);
-      else if (nT > 0) kAdjFace<R, true><<<RFLU_GRID(V, (long long)nT, s)>>>(V, W, 0, nT);
+      if (V.nb == 0 && nT > 0) interiorFaces(V, W, s);
+      else if (nT > 0) kAdjFace<R, 0><<<RFLU_GRID(V, (long long)nT, s)>>>(V, W, 0, nT);
       return;
     }
     SideStream &ss = sideStream();
     cudaEventRecord(ss.fork, s);
     cudaStreamWaitEvent(ss.stream, ss.fork, 0);
-    kAdjFace<R, false><<<RFLU_GRID(V, (long long)V.nb, ss.stream)>>>(V, W, V.nf, nT);
+    kAdjFace<R, 0><<<RFLU_GRID(V, (long long)V.nb, ss.stream)>>>(V, W, V.nf, nT);
     cudaEventRecord(ss.join, ss.stream);
-    if (roe2) kAdjFace<R, true><<<RFLU_GRID(V, (long long)V.nf, s)>>>(V, W, 0, V.nf);
-    else kAdjFace<R, false><<<RFLU_GRID(V, (long long)V.nf, s)>>>(V, W, 0, V.nf);
+    interiorFaces(V, W, s);
     cudaStreamWaitEvent(s, ss.join, 0);
   }
   static void vjp(const View<R> &V, const double *rhsBarRef, double *cvBarRef, double *work, cudaStream_t s) {

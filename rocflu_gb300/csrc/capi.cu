@@ -599,13 +599,14 @@ struct Ctx : CtxBase {
   // context that only steps does not hold it.
   int ensureAdjoint() {
     if (work) return RFLU_OK;
-    int rc = alloc((char **)&work, workBytes);
-    if (rc) return rc;
-    if (tsWidthLazy > 0) {
+    int rc = RFLU_OK;
+    if (tsWidthLazy > 0 && !V.tsW) {
       if ((rc = alloc(&V.tsW, 4 * (size_t)tsWidthLazy * V.nc))) return rc;
       V.tsWidth = tsWidthLazy;
-      ops->adjointSetup(V, stream);
     }
+    if (!Layout<R>::packed && V.p.spaceOrder > 1 && !V.wSum && (rc = alloc(&V.wSum, 3 * (size_t)V.nc))) return rc;
+    if ((rc = alloc((char **)&work, workBytes))) return rc;  // last: its presence says that all of them are there
+    ops->adjointSetup(V, stream);
     return checkLaunch("adjoint set-up");
   }
   // the host state cv in the scratch state W (the adjoint kernels then run on W)

@@ -141,6 +141,7 @@ struct View {
   int2 *fxW;
   int *fxScale;
   int fxWidth;
+  R *wSum;                          // FP64 layouts: each cell's sum of them (3, nc), for the adjoint
   const double *vol;
   const R *epsq;                    // Venkatakrishnan eps^2 = (vol^(1/3))^3 per cell
   // mixed mode: the LSQ weights w_j = L d_j / |d_j|^2 of a cell share one

@@ -2230,6 +2230,23 @@ __global__ void kTsWeights(View<R> V) {
   }
 }
 
+// The sum of each cell's least-squares weights (FP64 layouts, View::wSum).
+template <typename R>
+__global__ void __launch_bounds__(kBlock) kWeightSums(View<R> V) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= V.nc) return;
+  const size_t n = V.nc;
+  R x = R(0), y = R(0), z = R(0);
+  for (int s = V.stOff[i]; s < V.stOff[i + 1]; ++s) {
+    x = x + V.wx[s];
+    y = y + V.wy[s];
+    z = z + V.wz[s];
+  }
+  V.wSum[i] = x;
+  V.wSum[n + i] = y;
+  V.wSum[2 * n + i] = z;
+}
+
 // Time step alone from the primitive state (mixed mode).
 template <typename R>
 __global__ void __launch_bounds__(kBlock) kCellDtPrim(View<R> V) {
@@ -3032,6 +3049,9 @@ struct Launch {
   // Kernel attributes that depend on the mesh (shared memory of the tiled
   // kernels); called once at set-up, outside any stream capture.
   static void adjointSetup(const View<R> &V, cudaStream_t s) {
+    if constexpr (!Layout<R>::packed) {
+      if (V.wSum) kWeightSums<R><<<RFLU_GRID(V, V.nc, s)>>>(V);
+    }
     if (V.tsW) kTsWeights<R><<<RFLU_GRID(V, V.nc, s)>>>(V);
   }
   static void configure(const View<R> &V) {

@@ -101,3 +101,31 @@ def test_fixed_point_gradients(gpu_lib, mesh, state):
     prim = np.stack([rho, u[:, 0], u[:, 1], u[:, 2], p], axis=1)
     scale = np.abs(prim).max(axis=0) / h
     assert (np.abs(g - ref).max(axis=2) / np.maximum(scale, 1e-300)).max() < 1e-14
+
+
+@pytest.mark.parametrize("mesh", ["hex", "tets", "symmetry", "constrained", "periodic"])
+@pytest.mark.parametrize("reconst", [cases.RECONST_NONE, cases.RECONST_BJ_COMP, cases.RECONST_VENKAT,
+                                     cases.RECONST_BJ, cases.RECONST_WENO_XYZ])
+def test_tangent_and_adjoint_of_the_fixed_sums(gpu_lib, mesh, reconst):
+    """The fp64 mode's tangent (along the recorded branch) and adjoint against
+    the FP64_EXACT mode's (dual numbers, FP64 sums): the same linear maps, to
+    rounding amplified by the limiters' quotients."""
+    num = cases.Numerics(space_order=2, space_discr=cases.DISCR_HLLC, reconst=reconst, cfl=0.4)
+    if mesh == "tets":
+        c = cases.adjoint_tets(4, num=num)
+    elif mesh == "symmetry":
+        c = cases.mirror_box(5, axes=(0, 1, 2), num=num)
+    elif mesh == "periodic":
+        c = cases.gas_jump_periodic(5, left=(1.2, 0.0, 1.0), right=(0.97, 0.8))
+        c.num = num
+    else:
+        c = cases.shock_sphere(6, num=num)
+    if mesh == "constrained":
+        c.num.c_reconst = 1
+    c.cv0 = _wavy(c, amp=0.02)
+    rng = np.random.default_rng(2)
+    dot, bar = rng.standard_normal(c.cv0.shape), rng.standard_normal(c.cv0.shape)
+    a, b = gpu.Region(c, "fp64"), gpu.Region(c, "fp64_exact")
+    for x, y in ((a.jvp(c.cv0, dot), b.jvp(c.cv0, dot)), (a.vjp(c.cv0, bar), b.vjp(c.cv0, bar))):
+        assert np.isfinite(y).all()
+        assert np.abs(x - y).max() <= 1e-9 * np.abs(y).max()
