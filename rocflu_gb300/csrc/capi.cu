@@ -1613,8 +1613,8 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   workBytes = sizeof(R) * (size_t)(130 * (size_t)nc + 24 * ((size_t)nf + nb) + 64) + sizeof(int) * 10 * (size_t)nc + 256;
   ops->configure(V);
   RFLU_CUDA(cudaDeviceSynchronize());
-  V.tileGrid = ops->tileGrid(V, 0);
-  V.tileGridDt = ops->tileGrid(V, 1);
+  V.tileGrid = ops->tileGrid(V, 0, &V.tileBufs);
+  V.tileGridDt = ops->tileGrid(V, 1, &V.tileBufsDt);
   return checkLaunch("rflu_gpu_create");
 }
 

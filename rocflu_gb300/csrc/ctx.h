@@ -172,6 +172,7 @@ struct View {
   int tsWidth;                      // entries per cell of tsW
   int tileGrid;                     // CTAs of the persistent tiled kernels
   int tileGridDt;                   // ... of the variant with the time-step sum
+  int tileBufs, tileBufsDt;         // their tile buffers per CTA (1 or 2)
   int cfW;                          // max faces per cell (entries of feD/feN)
   const int *haloOff, *haloIdx;     // CSR over tiles of global halo cell ids by slot (-1: unused);
                                     // each tile's list starts on a 16-byte boundary
