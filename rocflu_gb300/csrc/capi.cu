@@ -1584,6 +1584,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   P.spaceOrder = num->spaceOrder; P.spaceDiscr = num->spaceDiscr; P.reconst = num->reconst;
   P.rkScheme = num->rkScheme; P.piclBuild = num->piclBuild; P.precision = num->precision;
   P.refCp = num->cp; P.refGamma = num->gamma;
+  P.refG1 = num->gamma - 1.0; P.refIg1 = 1.0 / P.refG1; P.refKh = num->cp / (num->cp - num->cp / num->gamma);
   P.gvCp = num->cp;
   P.gvMol = 8314.3 / (num->cp - num->cp / num->gamma);  // MixtPerf_M_R(MixtPerf_R_CpG(cp,gamma))
   P.gcR = 8314.3 / P.gvMol;                             // MixtPerf_R_M(M), the round trip

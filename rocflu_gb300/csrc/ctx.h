@@ -25,6 +25,7 @@ struct Scalars {
 struct Params {
   int spaceOrder, spaceDiscr, reconst, rkScheme, piclBuild, precision;
   double refCp, refGamma;     // global%refCp, global%refGamma (flux routines)
+  double refG1, refIg1, refKh;  // refGamma - 1, its reciprocal, refCp over the gas constant refCp - refCp/refGamma
   double gvCp, gvMol;         // gv(GV_MIXT_CP), gv(GV_MIXT_MOL) = 8314.3/R
   double gcR, gRT, igcR;      // 8314.3/gvMol, gvCp/(gvCp-gcR), 1/gcR (computed once on the host)
   // FP32 copies for the mixed-mode flux arithmetic (no per-face conversions)

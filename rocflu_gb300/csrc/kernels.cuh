@@ -22,6 +22,7 @@
 #include "dual.cuh"
 #include "fixedsum.h"
 #include "physics.cuh"
+#include "flux_fp64.cuh"
 
 namespace rflu {
 namespace RFLU_NS {
@@ -49,6 +50,16 @@ inline Shape shapeFor(const View<R> &V, long long n) {
   return shapeFor(V.sms, n);
 }
 #define RFLU_GRID(V, n, stream) shapeFor(V, n).grid, shapeFor(V, n).block, 0, stream
+
+// RFLU_PREC_FP64 (kernels_fp64.cu): the least-squares sums on the integer pipe
+// and the interior fluxes in their short form; the other modes compile neither.
+#ifdef RFLU_FIXED_SUMS
+constexpr bool kFixedSums = true;
+#else
+constexpr bool kFixedSums = false;
+#endif
+template <typename S>
+constexpr bool shortFlux() { return kFixedSums && std::is_same<S, double>::value; }
 
 // Reference arithmetic (the FP64 modes) reproduces the cons -> prim -> cons
 // round trip of CellGradientsMP on the fly; the mixed mode uses the
@@ -1350,11 +1361,6 @@ __device__ inline void cpAsync8(void *smemDst, const void *gSrc) {
 // than kFixMaxTerms members) run the FP64 loop.  FP64_EXACT keeps the FP64
 // loop for its bits, the mixed mode its FP32 sums.
 // ---------------------------------------------------------------------------
-#ifdef RFLU_FIXED_SUMS
-constexpr bool kFixedSums = true;
-#else
-constexpr bool kFixedSums = false;
-#endif
 constexpr int kFixBlock = 128;
 constexpr int kFixDepth = 8;  // members in flight per thread (a power of two)
 
@@ -2341,7 +2347,7 @@ __device__ inline void faceState(const View<R> &V, const L &ld, int c, typename 
   S r = q[0];
   S ir = div_(S(1), r);
   S u = q[1], v = q[2], w = q[3];
-  if (Ref<R>::on) {
+  if (Ref<R>::on && !shortFlux<S>()) {
     // ul = pCv(CV_MIXT_XMOM,c1)*irl with pCv(XMOM) = r*u after RFLU_ConvertCvPrim2Cons
     u = (r * u) * ir;
     v = (r * v) * ir;
@@ -2362,6 +2368,26 @@ template <> __device__ inline float prm<float>(double, float f) { return f; }
 
 template <typename S>
 __device__ inline void riemann2(const Params &P, S nx, S ny, S nz, S nm, const S *L, S irl, const S *Rt, S irr, S *flx) {
+  if constexpr (shortFlux<S>()) {
+    const double g = P.refGamma, il = div_(1.0, L[0]), ir = div_(1.0, Rt[0]);
+    const double tl = L[4] * il, tr = Rt[4] * ir;  // p / rho
+    const double kl = 0.5 * (L[1] * L[1] + L[2] * L[2] + L[3] * L[3]);
+    const double kr = 0.5 * (Rt[1] * Rt[1] + Rt[2] * Rt[2] + Rt[3] * Rt[3]);
+    if (P.spaceDiscr == 3) {
+      const double el = tl * P.refIg1 + kl, er = tr * P.refIg1 + kr;
+      hllcFluxShort(P.refG1, nx, ny, nz, nm, L[0], L[1], L[2], L[3], L[4], el, sqrt_(g * tl), el + irl * L[4], il,
+                    Rt[0], Rt[1], Rt[2], Rt[3], Rt[4], er, sqrt_(g * tr), er + irr * Rt[4], flx);
+      return;
+    }
+    const double Hl = P.refKh * tl + kl, Hr = P.refKh * tr + kr;
+    if (P.spaceDiscr == 1)
+      roeFluxShort(P.refG1, P.epsEntr, P.dissFact, nx, ny, nz, nm, L[0], L[1], L[2], L[3], L[4], Hl, Rt[0], Rt[1],
+                   Rt[2], Rt[3], Rt[4], Hr, flx);
+    else
+      ausmFluxShort(nx, ny, nz, nm, L[0], L[1], L[2], L[3], L[4], Hl, sqrt_(g * tl), Rt[0], Rt[1], Rt[2], Rt[3],
+                    Rt[4], Hr, sqrt_(g * tr), flx);
+    return;
+  }
   const S cp = prm<S>(P.refCp, P.refCpF), g = prm<S>(P.refGamma, P.refGammaF);
   if (P.spaceDiscr == 1) {
     S gc = cp - div_(cp, g);
@@ -2391,6 +2417,21 @@ __device__ inline void riemann1(const Params &P, const H *cl, const H *dvl, cons
   H rl = cl[0], irl = div_(H(1), rl), ul = cl[1] * irl, vl = cl[2] * irl, wl = cl[3] * irl;
   H rr = cr[0], irr = div_(H(1), rr), ur = cr[1] * irr, vr = cr[2] * irr, wr = cr[3] * irr;
   H pl = dvl[0], pr = dvr[0];
+  if constexpr (shortFlux<H>()) {
+    if (P.spaceDiscr == 1) {
+      roeFluxShort(P.refG1, P.epsEntr, P.dissFact, nx, ny, nz, nm, rl, ul, vl, wl, pl,
+                   perfHo(P.refCp, dvl[1], ul, vl, wl), rr, ur, vr, wr, pr, perfHo(P.refCp, dvr[1], ur, vr, wr), flx);
+      return;
+    }
+    const double el = cl[4] * irl, er = cr[4] * irr;
+    const double Hl = el + irl * pl, Hr = er + irr * pr;
+    if (P.spaceDiscr == 3)
+      hllcFluxShort(P.refG1, nx, ny, nz, nm, rl, ul, vl, wl, pl, el, dvl[2], Hl, irl, rr, ur, vr, wr, pr, er, dvr[2],
+                    Hr, flx);
+    else
+      ausmFluxShort(nx, ny, nz, nm, rl, ul, vl, wl, pl, Hl, dvl[2], rr, ur, vr, wr, pr, Hr, dvr[2], flx);
+    return;
+  }
   const H cp = H(P.refCp), g = H(P.refGamma);
   if (P.spaceDiscr == 1) {
     H Hl = perfHo(cp, dvl[1], ul, vl, wl), Hr = perfHo(cp, dvr[1], ur, vr, wr);

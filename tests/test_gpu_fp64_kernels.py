@@ -129,3 +129,24 @@ def test_tangent_and_adjoint_of_the_fixed_sums(gpu_lib, mesh, reconst):
     for x, y in ((a.jvp(c.cv0, dot), b.jvp(c.cv0, dot)), (a.vjp(c.cv0, bar), b.vjp(c.cv0, bar))):
         assert np.isfinite(y).all()
         assert np.abs(x - y).max() <= 1e-9 * np.abs(y).max()
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("discr", [cases.DISCR_ROE, cases.DISCR_HLLC, cases.DISCR_AUSM])
+@pytest.mark.parametrize("mach", [0.0, 0.4, -2.5, 2.5])
+def test_short_fluxes(gpu_lib, order, discr, mach):
+    """The fp64 mode's interior fluxes against the FP64_EXACT ones, with the
+    flow at rest, subsonic and supersonic either way: 1e-12 of each residual
+    component's largest value."""
+    num = cases.Numerics(space_order=order, space_discr=discr, reconst=0, cfl=0.4)
+    c = cases.blast_hex(7, num=num)
+    for p in c.patches:
+        p.order = order
+    rng = np.random.default_rng(8)
+    n = len(c.cv0)
+    rho, p = 1.0 + 0.2 * rng.random(n), 1.0 + 0.2 * rng.random(n)
+    u = (mach * np.sqrt(1.4) + 0.05 * rng.standard_normal(n), 0.05 * rng.standard_normal(n), 0.05 * rng.standard_normal(n))
+    c.cv0 = cases.conserved(rho, *u, p, c.num.gamma)
+    a, _ = gpu.Region(c, "fp64").residual(c.cv0, with_grad=False)
+    b, _ = gpu.Region(c, "fp64_exact").residual(c.cv0, with_grad=False)
+    assert (np.abs(a - b) / np.abs(b).max(axis=0)).max() < 1e-12
