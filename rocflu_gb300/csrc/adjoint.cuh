@@ -242,6 +242,7 @@ struct TanLoad {
 // ---------------------------------------------------------------------------
 template <typename R>
 __global__ void kTanInit(View<R> V, AdjWork<R> W, const double *cvDotRef) {
+  gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const size_t n = V.nc;
@@ -266,6 +267,7 @@ __global__ void kTanInit(View<R> V, AdjWork<R> W, const double *cvDotRef) {
 // hold an idle eigen-frame axis at the same factor).
 template <typename R>
 __global__ void __launch_bounds__(kBlock) kTanGrad(View<R> V, AdjWork<R> W, bool haveG) {
+  gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   Dual<1, R> g[15];
@@ -322,6 +324,7 @@ __device__ inline S venkat(S dext, S d2, S epsq) {
 // derivatives and run on dual numbers here.
 template <typename R>
 __global__ void __launch_bounds__(kBlock) kTanLimit(View<R> V, AdjWork<R> W) {
+  gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const size_t n = V.nc;
@@ -423,6 +426,7 @@ __device__ inline void wenoPositivity(const View<R> &V, int i, S *g, R *f0, R *f
 // (W.G, W.Gbar, written by kTanGrad), then the simple limiter.
 template <typename R>
 __global__ void __launch_bounds__(kBlock) kTanWeno(View<R> V, AdjWork<R> W) {
+  gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   using S = Dual<1, R>;
@@ -456,6 +460,7 @@ __global__ void __launch_bounds__(kBlock) kTanWeno(View<R> V, AdjWork<R> W) {
 
 template <typename R>
 __global__ void __launch_bounds__(kBlock) kTanFlux(View<R> V, AdjWork<R> W) {
+  gridOrder();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nT = V.nf + V.nb;
   if (t >= nT) return;
@@ -469,6 +474,7 @@ __global__ void __launch_bounds__(kBlock) kTanFlux(View<R> V, AdjWork<R> W) {
 
 template <typename R>
 __global__ void kTanGather(View<R> V, AdjWork<R> W, double *outRef) {
+  gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   R r[5];
@@ -483,6 +489,7 @@ __global__ void kTanGather(View<R> V, AdjWork<R> W, double *outRef) {
 // ---------------------------------------------------------------------------
 template <typename R>
 __global__ void kAdjLambda(View<R> V, AdjWork<R> W, const double *lamRef) {
+  gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const int o = V.refId[i];
@@ -781,6 +788,7 @@ __device__ inline void velFrameReverse(const View<R> &V, const L &ld, int i, con
 // haveG: W.G already holds the unlimited gradient (the fixed-point sums).
 template <typename R, bool kVel>
 __global__ void __launch_bounds__(kBlock) kAdjGradFwd(View<R> V, AdjWork<R> W, const double *lamRef, bool haveG) {
+  gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const size_t n = V.nc;
@@ -986,6 +994,7 @@ __device__ inline void wenoFwdFinish(const View<R> &V, AdjWork<R> &W, int i, R *
 // cell; simple form: 5).
 template <typename R>
 __global__ void __launch_bounds__(kBlock) kAdjWenoFwd(View<R> V, AdjWork<R> W) {
+  gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const size_t n = V.nc;
@@ -1015,6 +1024,7 @@ __global__ void __launch_bounds__(kBlock) kAdjWenoFwd(View<R> V, AdjWork<R> W) {
 // the ones of wenoXyz / wenoSimple, summed in another order).
 template <typename R>
 __global__ void __launch_bounds__(kBlock) kAdjWenoFwdLanes(View<R> V, AdjWork<R> W) {
+  gridOrder();
   if constexpr (Layout<R>::packed) {
     constexpr int kL = adjLanes<R>();
     const int th = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1125,6 +1135,7 @@ __device__ inline void contract(const Dual<N, T> *flx, const T *fbar, T *out) {
 // unrolled gradient 2.85 -> 2.53 ms.
 template <typename R, int kFlux>
 __global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int t0, int t1) {
+  gridOrder();
   const int t = t0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= t1) return;
   const Params &P = V.p;
@@ -1334,6 +1345,7 @@ __device__ inline void adjOwnTerm(const View<R> &V, const AdjWork<R> &W, int i, 
 
 template <typename R, bool kVel>
 __global__ void __launch_bounds__(kBlock) kAdjCell1(View<R> V, AdjWork<R> W) {
+  gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const Params &P = V.p;
@@ -1586,6 +1598,7 @@ __global__ void __launch_bounds__(kBlock) kAdjCell1(View<R> V, AdjWork<R> W) {
 // cell's primitive adjoint, and tbar for kAdjCell2's neighbour terms.
 template <typename R>
 __global__ void __launch_bounds__(kBlock) kAdjWeno(View<R> V, AdjWork<R> W) {
+  gridOrder();
   constexpr int kL = adjLanes<R>();  // lanes per cell for the gather
   const int th = blockIdx.x * blockDim.x + threadIdx.x;
   const int m = th / kL, h = th % kL;
@@ -1707,6 +1720,7 @@ __global__ void __launch_bounds__(kBlock) kAdjWeno(View<R> V, AdjWork<R> W) {
 // Neighbour terms, then (prim, dv) -> cv; output in reference order.
 template <typename R>
 __global__ void __launch_bounds__(kBlock) kAdjCell2(View<R> V, AdjWork<R> W, double *outRef) {
+  gridOrder();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= V.nc) return;
   const size_t n = V.nc;
@@ -1921,6 +1935,7 @@ __global__ void __launch_bounds__(kBlock) kAdjCell2(View<R> V, AdjWork<R> W, dou
 // these branches is a smooth function of the state.
 template <typename R>
 __global__ void kLimiterBranches(View<R> V, AdjWork<R> W, int *outRef) {
+  gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const size_t n = V.nc;
@@ -1960,6 +1975,7 @@ __global__ void kLimiterBranches(View<R> V, AdjWork<R> W, int *outRef) {
 // reduction.
 template <typename R>
 __global__ void kPatchSeed(View<R> V, AdjWork<R> W, int ip, double *Jout) {
+  gridOrder();
   __shared__ double part[kBlock];
   const size_t nb = V.nb;
   const PlainLoad<R> ld{V};
@@ -2012,47 +2028,48 @@ struct AdjointOps {
   static void jvp(const View<R> &V, const double *cvDotRef, double *rhsDotRef, double *work, cudaStream_t s) {
     const size_t nT = (size_t)V.nf + V.nb;
     AdjWork<R> W = carveAdjWork<R>(work, V.nc, nT);
-    kTanInit<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, cvDotRef);
+    launchOrdered(kTanInit<R>, shapeFor(V, V.nc), s, V, W, cvDotRef);
     const int rc = V.p.reconst;
     if (Launch<R>::fixedSums(V) && (rc == 0 || rc == 100 || rc == 11)) {
       gradFwd(V, W, nullptr, s);
       Launch<R>::launchFixed(V, W.primd, W.Gbar, false, s);
-      kTanLimit<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
+      launchOrdered(kTanLimit<R>, shapeFor(V, V.nc), s, V, W);
     } else if (V.p.spaceOrder > 1) {
       const bool haveG = Launch<R>::fixedSums(V);
       if (haveG) {
         Launch<R>::launchFixed(V, V.prim, W.G, true, s);
         Launch<R>::launchFixed(V, W.primd, W.Gbar, false, s);
       }
-      kTanGrad<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, haveG);
+      launchOrdered(kTanGrad<R>, shapeFor(V, V.nc), s, V, W, haveG);
     }
-    if (isWeno(V.p)) kTanWeno<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
-    kTanFlux<R><<<RFLU_GRID(V, (long long)nT, s)>>>(V, W);
-    kTanGather<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, rhsDotRef);
+    if (isWeno(V.p)) launchOrdered(kTanWeno<R>, shapeFor(V, V.nc), s, V, W);
+    launchOrdered(kTanFlux<R>, shapeFor(V, (long long)nT), s, V, W);
+    launchOrdered(kTanGather<R>, shapeFor(V, V.nc), s, V, W, rhsDotRef);
   }
   static void gradFwd(const View<R> &V, const AdjWork<R> &W, const double *lamRef, cudaStream_t s) {
     const bool haveG = Launch<R>::fixedSums(V);
     if (haveG) Launch<R>::launchFixed(V, V.prim, W.G, true, s);
-    if (V.p.reconst == 10) kAdjGradFwd<R, true><<<RFLU_GRID(V, V.nc, s)>>>(V, W, lamRef, haveG);
-    else kAdjGradFwd<R, false><<<RFLU_GRID(V, V.nc, s)>>>(V, W, lamRef, haveG);
+    if (V.p.reconst == 10) launchOrdered(kAdjGradFwd<R, true>, shapeFor(V, V.nc), s, V, W, lamRef, haveG);
+    else launchOrdered(kAdjGradFwd<R, false>, shapeFor(V, V.nc), s, V, W, lamRef, haveG);
     if (isWeno(V.p)) {
       if constexpr (Layout<R>::packed)
-        kAdjWenoFwdLanes<R><<<RFLU_GRID(V, (long long)V.nc * adjLanes<R>(), s)>>>(V, W);
+        launchOrdered(kAdjWenoFwdLanes<R>, shapeFor(V, (long long)V.nc * adjLanes<R>()), s, V, W);
       else
-        kAdjWenoFwd<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
+        launchOrdered(kAdjWenoFwd<R>, shapeFor(V, V.nc), s, V, W);
     }
   }
   static void cellAdjoint(const View<R> &V, AdjWork<R> &W, double *cvBarRef, cudaStream_t s) {
-    if (V.p.reconst == 10 && V.p.spaceOrder > 1) kAdjCell1<R, true><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
-    else kAdjCell1<R, false><<<RFLU_GRID(V, V.nc, s)>>>(V, W);
-    if (isWeno(V.p)) kAdjWeno<R><<<RFLU_GRID(V, (long long)V.nc * adjLanes<R>(), s)>>>(V, W);
-    kAdjCell2<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, cvBarRef);
+    const Shape sh = shapeFor(V, V.nc);  // after the side stream's event: launched plainly
+    if (V.p.reconst == 10 && V.p.spaceOrder > 1) kAdjCell1<R, true><<<sh.grid, sh.block, 0, s>>>(V, W);
+    else kAdjCell1<R, false><<<sh.grid, sh.block, 0, s>>>(V, W);
+    if (isWeno(V.p)) launchOrdered(kAdjWeno<R>, shapeFor(V, (long long)V.nc * adjLanes<R>()), s, V, W);
+    launchOrdered(kAdjCell2<R>, shapeFor(V, V.nc), s, V, W, cvBarRef);
   }
   static void interiorFaces(const View<R> &V, const AdjWork<R> &W, cudaStream_t s) {
     const int flux = V.p.spaceOrder > 1 ? V.p.spaceDiscr : 0;
-    if (flux == 1) kAdjFace<R, 1><<<RFLU_GRID(V, (long long)V.nf, s)>>>(V, W, 0, V.nf);
-    else if (flux == 3) kAdjFace<R, 3><<<RFLU_GRID(V, (long long)V.nf, s)>>>(V, W, 0, V.nf);
-    else kAdjFace<R, 0><<<RFLU_GRID(V, (long long)V.nf, s)>>>(V, W, 0, V.nf);
+    if (flux == 1) launchOrdered(kAdjFace<R, 1>, shapeFor(V, (long long)V.nf), s, V, W, 0, V.nf);
+    else if (flux == 3) launchOrdered(kAdjFace<R, 3>, shapeFor(V, (long long)V.nf), s, V, W, 0, V.nf);
+    else launchOrdered(kAdjFace<R, 0>, shapeFor(V, (long long)V.nf), s, V, W, 0, V.nf);
   }
   // The boundary faces' kernel (dual numbers through the patch fluxes; few
   // faces, a small grid) runs on a second stream beside the interior faces'
@@ -2063,13 +2080,14 @@ struct AdjointOps {
     const int nT = V.nf + V.nb;
     if (V.nf == 0 || V.nb == 0) {
       if (V.nb == 0 && nT > 0) interiorFaces(V, W, s);
-      else if (nT > 0) kAdjFace<R, 0><<<RFLU_GRID(V, (long long)nT, s)>>>(V, W, 0, nT);
+      else if (nT > 0) launchOrdered(kAdjFace<R, 0>, shapeFor(V, (long long)nT), s, V, W, 0, nT);
       return;
     }
     SideStream &ss = sideStream();
     cudaEventRecord(ss.fork, s);
     cudaStreamWaitEvent(ss.stream, ss.fork, 0);
-    kAdjFace<R, 0><<<RFLU_GRID(V, (long long)V.nb, ss.stream)>>>(V, W, V.nf, nT);
+    const Shape sh = shapeFor(V, (long long)V.nb);  // after an event: launched plainly
+    kAdjFace<R, 0><<<sh.grid, sh.block, 0, ss.stream>>>(V, W, V.nf, nT);
     cudaEventRecord(ss.join, ss.stream);
     interiorFaces(V, W, s);
     cudaStreamWaitEvent(s, ss.join, 0);
@@ -2080,7 +2098,7 @@ struct AdjointOps {
     // every face-adjoint entry the cell kernels read is written by the face
     // kernels: no clearing of faceAdj here
     if (V.p.spaceOrder > 1) gradFwd(V, W, rhsBarRef, s);
-    else kAdjLambda<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, rhsBarRef);
+    else launchOrdered(kAdjLambda<R>, shapeFor(V, V.nc), s, V, W, rhsBarRef);
     (void)nT;
     faceAdjoint(V, W, s);
     cellAdjoint(V, W, cvBarRef, s);
@@ -2089,7 +2107,7 @@ struct AdjointOps {
     const size_t nT = (size_t)V.nf + V.nb;
     AdjWork<R> W = carveAdjWork<R>(work, V.nc, nT);
     gradFwd(V, W, nullptr, s);
-    kLimiterBranches<R><<<RFLU_GRID(V, V.nc, s)>>>(V, W, outRef);
+    launchOrdered(kLimiterBranches<R>, shapeFor(V, V.nc), s, V, W, outRef);
   }
   static void patchPressure(const View<R> &V, int ip, double *J, double *cvBarRef, double *work, cudaStream_t s) {
     const size_t nT = (size_t)V.nf + V.nb;
