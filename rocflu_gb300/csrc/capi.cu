@@ -342,8 +342,10 @@ struct Ctx : CtxBase {
   Scalars *sSc = nullptr;
   cudaGraphExec_t stepGraph = nullptr, fixedGraph = nullptr;
   long long lastNan = 0;
+  Scalars *hostSc = nullptr;  // pinned copy of V.sc (readScalars)
 
   ~Ctx() override {
+    if (hostSc) cudaFreeHost(hostSc);
     if (stepGraph) cudaGraphExecDestroy(stepGraph);
     if (fixedGraph) cudaGraphExecDestroy(fixedGraph);
     for (void *p : allocs) cudaFree(p);
@@ -403,11 +405,25 @@ struct Ctx : CtxBase {
     if (e != cudaSuccess) return fail(RFLU_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
     return RFLU_OK;
   }
-  int syncEvents(bool events) {
+  // The context's scalars after everything queued on the stream, through a
+  // pinned copy: one wait (a pageable copy and a second wait for it cost
+  // another 10-15 us per stage of a host-driven loop).
+  int readScalars(Scalars *s) {
+    RFLU_CUDA(cudaMemcpyAsync(hostSc, V.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream));
     RFLU_CUDA(cudaStreamSynchronize(stream));
-    if (!events) return RFLU_OK;
+    *s = *hostSc;
+    return RFLU_OK;
+  }
+  int syncEvents(bool events) {
+    if (!events) {
+      RFLU_CUDA(cudaStreamSynchronize(stream));
+      return RFLU_OK;
+    }
     Scalars s;
-    RFLU_CUDA(cudaMemcpy(&s, V.sc, sizeof(Scalars), cudaMemcpyDeviceToHost));
+    if (int rc = readScalars(&s)) return rc;
+    return eventOf(s);
+  }
+  int eventOf(const Scalars &s) {
     if ((long long)s.nanCells > lastNan) {
       lastNan = (long long)s.nanCells;
       return RFLU_EVENT_NAN;
@@ -512,8 +528,7 @@ struct Ctx : CtxBase {
     int rc = checkLaunch("timestep");
     if (rc) return rc;
     Scalars s;
-    RFLU_CUDA(cudaMemcpyAsync(&s, V.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream));
-    RFLU_CUDA(cudaStreamSynchronize(stream));
+    if ((rc = readScalars(&s))) return rc;
     if (dt) *dt = s.dtMin;
     return RFLU_OK;
   }
@@ -573,16 +588,14 @@ struct Ctx : CtxBase {
       int m = std::min(chunk, nSteps - n0);
       for (int k = 0; k < m; ++k) RFLU_CUDA(cudaGraphLaunch(stepGraph, stream));
       if (endTime > 0.0) {
-        RFLU_CUDA(cudaMemcpyAsync(&s, V.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream));
-        RFLU_CUDA(cudaStreamSynchronize(stream));
+        if ((rc = readScalars(&s))) return rc;
         if (s.finished != 0) break;
       }
     }
-    RFLU_CUDA(cudaMemcpyAsync(&s, V.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream));
-    rc = syncEvents(true);
+    if ((rc = readScalars(&s))) return rc;
     *time = s.time;
     if (done) *done = s.stepsDone;
-    return rc;
+    return eventOf(s);
   }
   int runFixedDt(int nSteps, double dt) override {
     invalidate();
@@ -789,8 +802,7 @@ struct Ctx : CtxBase {
 
   int status(rflu_status *st) override {
     Scalars s;
-    RFLU_CUDA(cudaStreamSynchronize(stream));
-    RFLU_CUDA(cudaMemcpy(&s, V.sc, sizeof(Scalars), cudaMemcpyDeviceToHost));
+    if (int rc = readScalars(&s)) return rc;
     st->nanCells = (long long)s.nanCells;
     st->posFixCells = (long long)s.posFixCells;
     st->negPCells = (long long)s.negPCells;
@@ -1594,6 +1606,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   if ((rc = alloc(&V.flux, 5 * ((size_t)nf + nb)))) return rc;
   if ((rc = alloc(&V.rhs, 5 * (size_t)nc))) return rc;
   if ((rc = alloc(&V.sc, 1))) return rc;
+  RFLU_CUDA(cudaMallocHost((void **)&hostSc, sizeof(Scalars)));
   if ((rc = alloc(&staging, 15 * (size_t)nc + 16))) return rc;
   RFLU_CUDA(cudaMemset(V.grad, 0, sizeof(R) * Layout<R>::grad * (size_t)nc));
   RFLU_CUDA(cudaMemset(V.rhsSum, 0, sizeof(R) * 5 * (size_t)nc));
