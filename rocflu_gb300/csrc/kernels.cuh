@@ -978,6 +978,52 @@ __device__ inline float tileDtSum(const View<float> &V, int i, const float *recs
   return sum;
 }
 
+// Eigenvalues (ascending) and eigenvectors (columns) of the strain rate in
+// FP32: cyclic Jacobi rotations as symmetricEigen3 takes them, each angle's
+// tangent as b / (d + sgn(d) sqrt(d^2 + b^2)), d = r_qq - r_pp, b = 2 r_pq (one
+// root, one reciprocal and one reciprocal root, about 40 instructions a
+// rotation instead of 60), until the off-diagonals are below 2^-25 of the
+// matrix, half a rounding of its FP32 entries; the general routine's 1e-12
+// costs a sweep more that turns the axes by less than that.  Measured with
+// every cell's frame active, 128^3: 10 steps 16.07 -> 15.74 ms.
+__device__ inline void strainFrame(const float *m, float *vec, float *val) {
+  float r0 = m[0], r1 = m[4], r2 = m[8], r01 = m[3], r02 = m[6], r12 = m[7];
+  const float total = r0 * r0 + r1 * r1 + r2 * r2 + 2.f * (r01 * r01 + r02 * r02 + r12 * r12);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) vec[k] = 0.f;
+  vec[0] = vec[4] = vec[8] = 1.f;
+  const float tol = 8.8e-16f * total;
+  // rotation in the plane of p and q; o the third axis
+  auto rotate = [&](float &pp, float &qq, float &pq, float &op, float &oq, float *vp, float *vq) {
+    const float d = qq - pp, b = 2.f * pq, h = d * d + b * b;
+    if (pq == 0.f || !(h > 0.f)) return;  // nothing to turn, or both squares underflow
+    const float t = __fdividef(b, d + copysignf(sqrtf(h), d));
+    const float c = rsqrtf(t * t + 1.f), s = t * c;
+    pp = pp - t * pq;
+    qq = qq + t * pq;
+    pq = 0.f;
+    const float a = op;
+    op = c * a - s * oq;
+    oq = s * a + c * oq;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float x = vp[k];
+      vp[k] = c * x - s * vq[k];
+      vq[k] = s * x + c * vq[k];
+    }
+  };
+  for (int sweep = 0; sweep < 50; ++sweep) {
+    if (r01 * r01 + r02 * r02 + r12 * r12 <= tol) break;
+    rotate(r0, r1, r01, r02, r12, vec, vec + 3);
+    rotate(r0, r2, r02, r01, r12, vec, vec + 6);
+    rotate(r1, r2, r12, r01, r02, vec + 3, vec + 6);
+  }
+  val[0] = r0;
+  val[1] = r1;
+  val[2] = r2;
+  sortAxes(val, vec);
+}
+
 template <bool kDt, bool kTiled, int kRc>
 __device__ inline float gradLimitPacked(const View<float> &V, int i, float *g, float *dc, const float *recs,
                                         int li, const unsigned short *stSm = nullptr,
@@ -1126,7 +1172,7 @@ __device__ inline float gradLimitPacked(const View<float> &V, int i, float *g, f
     for (int a = 0; a < 3; ++a)
 #pragma unroll
       for (int b = 0; b < 3; ++b) Sy[a + 3 * b] = 0.5f * (G[a + 3 * b] + G[b + 3 * a]);
-    symmetricEigen3(Sy, A, ev);
+    strainFrame(Sy, A, ev);
     float mx = fabsf(ev[0]);
     mx = fmax2(mx, fabsf(ev[1]));
     mx = fmax2(mx, fabsf(ev[2]));

@@ -407,6 +407,23 @@ __host__ __device__ inline void injectionPatchFlux(const double *K, S g, S cp, S
 // all five components (ConvectiveFluxes' patch loop).
 __host__ __device__ inline bool patchLeavesDensity(int type) { return type == 60 || type == 70 || type == 71; }
 
+// Selection sort of eigenvalues and eigenvector columns (first strict minimum,
+// swapped into place), written with fixed indices so that val and vec stay in
+// registers.
+template <typename S>
+__host__ __device__ inline void sortAxes(S val[3], S vec[9]) {
+  auto swapCols = [&](int a, int b) {
+    S t = val[a]; val[a] = val[b]; val[b] = t;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { S x = vec[k + 3 * a]; vec[k + 3 * a] = vec[k + 3 * b]; vec[k + 3 * b] = x; }
+  };
+  const bool m1 = less_(val[1], val[0]);
+  const bool m2 = less_(val[2], m1 ? val[1] : val[0]);
+  if (m2) swapCols(0, 2);
+  else if (m1) swapCols(0, 1);
+  if (less_(val[2], val[1])) swapCols(1, 2);
+}
+
 // Cyclic Jacobi eigen-decomposition of a symmetric 3x3 (RFLU_SymmetricEigen3,
 // modflu/RFLU_ModLimiters.F90:791-912): ascending eigenvalues, eigenvectors
 // as columns.  m, vec are column-major.
@@ -455,18 +472,7 @@ __host__ __device__ inline void symmetricEigen3(const S m[9], S vec[9], S val[3]
       }
   }
   val[0] = r[0]; val[1] = r[4]; val[2] = r[8];
-  // selection sort (first strict minimum, swapped into place), written with
-  // fixed indices so that val and vec stay in registers
-  auto swapCols = [&](int a, int b) {
-    S t = val[a]; val[a] = val[b]; val[b] = t;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) { S x = vec[k + 3 * a]; vec[k + 3 * a] = vec[k + 3 * b]; vec[k + 3 * b] = x; }
-  };
-  const bool m1 = less_(val[1], val[0]);
-  const bool m2 = less_(val[2], m1 ? val[1] : val[0]);
-  if (m2) swapCols(0, 2);
-  else if (m1) swapCols(0, 1);
-  if (less_(val[2], val[1])) swapCols(1, 2);
+  sortAxes(val, vec);
 }
 
 // Whether eigenvalues j < k (ascending) lie in one group of the eigen-frame
