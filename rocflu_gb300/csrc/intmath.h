@@ -73,6 +73,15 @@ RFLU_HD inline bool isLessEq(double a, double b) {
   return kx <= ky && mx <= inf && my <= inf;
 }
 
+// A double as an integer in the doubles' order (-0 just below +0; NaN beyond the
+// infinities), and back: minima and maxima of many values as integer ones.
+RFLU_HD inline int64_t orderKey(double x) {
+  const int64_t b = (int64_t)bitsOf(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+RFLU_HD inline double ofKey(int64_t k) { return ofBits((uint64_t)(k ^ ((k >> 63) & 0x7fffffffffffffffll))); }
+constexpr int64_t kKeyInf = 0x7ff0000000000000ll;  // orderKey(infinity); a NaN's key is above it or below -1 - it
+
 // The FP32 approximations the iterations start from, as 32-bit fractions of
 // an argument's significand: f has the leading 24 bits; results in (1/2, 1].
 RFLU_HD inline uint32_t seedFraction(float r) {

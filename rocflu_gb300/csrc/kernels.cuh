@@ -986,8 +986,7 @@ __device__ inline float tileDtSum(const View<float> &V, int i, const float *recs
 // matrix, half a rounding of its FP32 entries; the general routine's 1e-12
 // costs a sweep more that turns the axes by less than that.  Measured with
 // every cell's frame active, 128^3: 10 steps 16.07 -> 15.74 ms.
-__device__ inline void strainFrame(const float *m, float *vec, float *val) {
-  float r0 = m[0], r1 = m[4], r2 = m[8], r01 = m[3], r02 = m[6], r12 = m[7];
+__device__ inline void jacobi3(float &r0, float &r1, float &r2, float r01, float r02, float r12, float *vec) {
   const float total = r0 * r0 + r1 * r1 + r2 * r2 + 2.f * (r01 * r01 + r02 * r02 + r12 * r12);
 #pragma unroll
   for (int k = 0; k < 9; ++k) vec[k] = 0.f;
@@ -1018,9 +1017,12 @@ __device__ inline void strainFrame(const float *m, float *vec, float *val) {
     rotate(r0, r2, r02, r01, r12, vec, vec + 6);
     rotate(r1, r2, r12, r01, r02, vec + 3, vec + 6);
   }
-  val[0] = r0;
-  val[1] = r1;
-  val[2] = r2;
+}
+__device__ inline void strainFrame(const float *m, float *vec, float *val) {
+  val[0] = m[0];
+  val[1] = m[4];
+  val[2] = m[8];
+  jacobi3(val[0], val[1], val[2], m[3], m[6], m[7], vec);
   sortAxes(val, vec);
 }
 
@@ -1673,9 +1675,219 @@ __global__ void __launch_bounds__(kFixBlock, 3) kGradFixed(View<R> V, const R *q
   }
 }
 
+// Eigenvalues (ascending) and eigenvectors (columns) of a symmetric matrix in
+// RFLU_PREC_FP64, to symmetricEigen3's tolerance (off-diagonals below 1e-12 of
+// the matrix): the rotations run in FP32 on the scaled matrix first (jacobi3),
+// their product is orthonormalised in FP64 and the matrix turned by it, which
+// leaves off-diagonals near 1e-7, and one FP64 sweep of small angles ends it:
+// about 170 FP64 instructions instead of 90 per sweep and four or five sweeps.
+__device__ inline void strainFrame64(const double *m, double *vec, double *val) {
+  const double s00 = m[0], s11 = m[4], s22 = m[8], s01 = m[3], s02 = m[6], s12 = m[7];
+  auto expOf = [](double x) { return (int)(bitsOf(x) >> 52) & 0x7ff; };
+  const int e = max(max(max(expOf(s00), expOf(s11)), max(expOf(s22), expOf(s01))), max(expOf(s02), expOf(s12)));
+  if (e < 523 || e > 1523) {  // zero, or squares that leave the range
+    symmetricEigen3(m, vec, val);
+    return;
+  }
+  // in [0, 2) of the largest entry's power of two, cut to 24 bits
+  auto scaled = [&](double x) {
+    const uint64_t b = bitsOf(x);
+    const int k = expOf(x) - e + 127;
+    return k <= 0 ? 0.f
+                  : __uint_as_float((unsigned)(b >> 32) & 0x80000000u | (unsigned)k << 23 | (unsigned)(b >> 29) & 0x7fffffu);
+  };
+  float f0 = scaled(s00), f1 = scaled(s11), f2 = scaled(s22), vf[9];
+  jacobi3(f0, f1, f2, scaled(s01), scaled(s02), scaled(s12), vf);
+  double *a = vec, *b = vec + 3, *c = vec + 6;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) vec[k] = f2d(vf[k]);
+  // a, then b, orthonormal from near it: 1/sqrt(1 + x) = 1 - x/2 + 3 x^2/8
+  auto unit = [](double *v) {
+    const double x = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] - 1.0;
+    const double s = x * (0.375 * x - 0.5) + 1.0;
+    v[0] = v[0] * s;
+    v[1] = v[1] * s;
+    v[2] = v[2] * s;
+  };
+  unit(a);
+  const double ab = a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) b[k] = b[k] - ab * a[k];
+  unit(b);
+  c[0] = a[1] * b[2] - a[2] * b[1];
+  c[1] = a[2] * b[0] - a[0] * b[2];
+  c[2] = a[0] * b[1] - a[1] * b[0];
+  double r[3], r01, r02, r12;
+  {
+    auto times = [&](const double *v, double *y) {
+      y[0] = s00 * v[0] + s01 * v[1] + s02 * v[2];
+      y[1] = s01 * v[0] + s11 * v[1] + s12 * v[2];
+      y[2] = s02 * v[0] + s12 * v[1] + s22 * v[2];
+    };
+    auto dot = [](const double *x, const double *y) { return x[0] * y[0] + x[1] * y[1] + x[2] * y[2]; };
+    double y[3];
+    times(a, y);
+    r[0] = dot(a, y);
+    r01 = dot(b, y);
+    r02 = dot(c, y);
+    times(b, y);
+    r[1] = dot(b, y);
+    r12 = dot(c, y);
+    times(c, y);
+    r[2] = dot(c, y);
+  }
+  auto rotate = [](double &pp, double &qq, double &pq, double &op, double &oq, double *vp, double *vq) {
+    if (!nonZero_(pq)) return;
+    const double d = qq - pp;
+    double t, cs;
+    const int ed = (int)(bitsOf(d) >> 52) & 0x7ff, ep = (int)(bitsOf(pq) >> 52) & 0x7ff;
+    if (ed - ep >= 17) {  // |pq / d| < 2^-16: the angle's tangent to 2^-64 from its series
+      const double x = div_(pq, d);
+      t = x - x * (x * x);
+      cs = 1.0 - 0.5 * (t * t);
+    } else {
+      const double bb = 2.0 * pq;
+      t = div_(bb, d + copysign_(sqrt_(d * d + bb * bb), d));
+      cs = div_(1.0, sqrt_(t * t + 1.0));
+    }
+    const double sn = t * cs, x = op;
+    pp = pp - t * pq;
+    qq = qq + t * pq;
+    pq = 0.0;
+    op = cs * x - sn * oq;
+    oq = sn * x + cs * oq;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double y = vp[k];
+      vp[k] = cs * y - sn * vq[k];
+      vq[k] = sn * y + cs * vq[k];
+    }
+  };
+  const double tol = 1.0e-24 * (r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
+  for (int sweep = 0; sweep < 50; ++sweep) {
+    if (lessEq_(r01 * r01 + r02 * r02 + r12 * r12, tol)) break;
+    rotate(r[0], r[1], r01, r02, r12, a, b);
+    rotate(r[0], r[2], r02, r01, r12, a, c);
+    rotate(r[1], r[2], r12, r01, r02, b, c);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) val[k] = r[k];
+  sortAxes(val, vec);
+}
+
+// limitCell's Barth-Jespersen limiters (RECONST 10 and 100) for
+// RFLU_PREC_FP64, in one pass over the faces like gradLimitPacked: the
+// neighbours' extremes, the extreme projections of the face offsets and, in
+// the eigen-frame, of the velocity differences, all kept as integers in the
+// doubles' order; the frame's projections take B = A^T G, and a factor is
+// divided only where it limits.  Bound by the FP64 pipe.  Measured, 421,875
+// cells with every frame active: 2 steps 8.43 -> 6.10 ms.
+template <bool kVel, typename R>
+__device__ inline void limitCellShort(const View<R> &V, int i, const double *q, double *g) {
+  const PlainLoad<R> ld{V};
+  const size_t n = V.nc;
+  double A[9], B[9], ev[3];
+  if (kVel) {
+    double Sy[9];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b)
+        Sy[a + 3 * b] = a == b ? g[3 * (1 + a) + a] : 0.5 * (g[3 * (1 + a) + b] + g[3 * (1 + b) + a]);
+    strainFrame64(Sy, A, ev);
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) B[3 * j + c] = A[3 * j] * g[3 + c] + A[3 * j + 1] * g[6 + c] + A[3 * j + 2] * g[9 + c];
+  }
+  constexpr int kS = kVel ? 2 : 5;  // scalar variables: density and pressure, or all
+  int64_t vmin[kS], vmax[kS], pmx[kS], pmn[kS];
+  int64_t umin[3], umax[3], smx[3], smn[3];
+#pragma unroll
+  for (int s = 0; s < kS; ++s) {
+    vmin[s] = vmax[s] = orderKey(q[kVel ? 4 * s : s]);
+    pmx[s] = pmn[s] = 0;
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) umin[j] = umax[j] = smx[j] = smn[j] = 0;
+  // a NaN takes no part, as in the comparisons it fails
+  auto take = [](int64_t k, int64_t &lo, int64_t &hi) {
+    if (k > hi && k <= kKeyInf) hi = k;
+    if (k < lo && k >= -1 - kKeyInf) lo = k;
+  };
+  const int ce = V.cfOff[i + 1];
+  for (int e = V.cfOff[i]; e < ce; ++e) {
+    const int code = V.cfEnt[e];
+    double x[5], d[3];
+    if (code < 0) {
+      const double *Q = symmetryQ(V, code);
+      if (!Q) continue;
+      x[0] = q[0];
+      reflect3(Q, q + 1, x + 1);
+      x[4] = q[4];
+    } else {
+      const int f = code >> 1, nb = (code & 1) ? V.fc1[f] : V.fc2[f];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) x[k] = V.prim[k * n + nb];
+    }
+    limiterFaceOffset(V, code, d);
+#pragma unroll
+    for (int s = 0; s < kS; ++s) {
+      const int k = kVel ? 4 * s : s;
+      take(orderKey(x[k]), vmin[s], vmax[s]);
+      take(orderKey(-(g[3 * k] * d[0] + g[3 * k + 1] * d[1] + g[3 * k + 2] * d[2])), pmn[s], pmx[s]);
+    }
+    if (kVel) {
+      const double du[3] = {x[1] - q[1], x[2] - q[2], x[3] - q[3]};
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        take(orderKey(A[3 * j] * du[0] + A[3 * j + 1] * du[1] + A[3 * j + 2] * du[2]), umin[j], umax[j]);
+        take(orderKey(-(B[3 * j] * d[0] + B[3 * j + 1] * d[1] + B[3 * j + 2] * d[2])), smn[j], smx[j]);
+      }
+    }
+  }
+  // min(1, hi / largest, lo / smallest): a quotient of same-signed numbers
+  // limits where the numerator is the smaller
+  auto factor = [](double hi, double lo, int64_t largest, int64_t smallest) {
+    double l = 1.0;
+    const double p = ofKey(largest), m = ofKey(smallest);
+    if (largest > 0 && less_(hi, p)) l = div_(hi, p);
+    if (smallest < 0 && nonZero_(m) && less_(m, lo)) l = fmin2(div_(lo, m), l);
+    return l;
+  };
+#pragma unroll
+  for (int s = 0; s < kS; ++s) {
+    const int k = kVel ? 4 * s : s;
+    const double l = factor(ofKey(vmax[s]) - q[k], ofKey(vmin[s]) - q[k], pmx[s], pmn[s]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) g[3 * k + c] = l * g[3 * k + c];
+  }
+  if (kVel) {
+    double al[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) al[j] = factor(ofKey(umax[j]), ofKey(umin[j]), smx[j], smn[j]);
+    const double mx = fmax2(fmax2(fabs_(ev[0]), fabs_(ev[1])), fabs_(ev[2]));
+    const double scale = 1.0e-3 * mx;
+    const bool e12 = lessEq_(ev[1] - ev[0], scale), e23 = lessEq_(ev[2] - ev[1], scale);
+    const double a01 = fmin2(al[0], al[1]), a12 = fmin2(al[1], al[2]);
+    if (e12 && e23) al[0] = al[1] = al[2] = fmin2(a01, al[2]);
+    else if (e12) al[0] = al[1] = a01;
+    else if (e23) al[1] = al[2] = a12;
+    // G <- A diag(al) A^T G = A diag(al) B
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) B[3 * j + c] = al[j] * B[3 * j + c];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) g[3 * (1 + a) + c] = A[a] * B[c] + A[a + 3] * B[3 + c] + A[a + 6] * B[6 + c];
+  }
+}
+
 // The limiter alone, on the unlimited gradients in V.grad (FP64 layouts).
-template <typename R>
-__global__ void __launch_bounds__(kBlock) kLimit(View<R> V) {
+template <typename R, int kRc>
+__global__ void __launch_bounds__(kFixBlock) kLimit(View<R> V) {
   gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
@@ -1685,7 +1897,8 @@ __global__ void __launch_bounds__(kBlock) kLimit(View<R> V) {
   ld.prim5(i, q);
 #pragma unroll
   for (int k = 0; k < 15; ++k) g[k] = V.grad[k * n + i];
-  limitCell(V, ld, i, q, g);
+  if constexpr (kRc == 11) limitCell(V, ld, i, q, g);
+  else limitCellShort<kRc == 10>(V, i, q, g);
   storeGrad(V, i, g);
 }
 
@@ -3166,7 +3379,13 @@ struct Launch {
     }
   }
   static void launchLimit(const View<R> &V, cudaStream_t s) {
-    if constexpr (kFixedSums && !Layout<R>::packed) launchOrdered(kLimit<R>, shapeFor(V, V.nc), s, V);
+    if constexpr (kFixedSums && !Layout<R>::packed) {
+      const int b = std::min(kFixBlock, shapeFor(V, V.nc).block);
+      const Shape sh{(V.nc + b - 1) / b, b};
+      if (V.p.reconst == 10) launchOrdered(kLimit<R, 10>, sh, s, V);
+      else if (V.p.reconst == 100) launchOrdered(kLimit<R, 100>, sh, s, V);
+      else launchOrdered(kLimit<R, 11>, sh, s, V);
+    }
   }
   // FP64 layouts: one thread per cell and variable (blockIdx.y).  The
   // constrained gradients' rows run through a cell's variables in turn and
