@@ -1680,7 +1680,11 @@ __global__ void __launch_bounds__(kFixBlock, 3) kGradFixed(View<R> V, const R *q
 // the matrix): the rotations run in FP32 on the scaled matrix first (jacobi3),
 // their product is orthonormalised in FP64 and the matrix turned by it, which
 // leaves off-diagonals near 1e-7, and one FP64 sweep of small angles ends it:
-// about 170 FP64 instructions instead of 90 per sweep and four or five sweeps.
+// some 155 FP64 instructions, counted in the source, instead of 90 per sweep and
+// four or five sweeps.  What is left off the diagonal, of the matrix's norm and
+// in 128-bit arithmetic over 400,000 normal matrices: median 3e-16, 99 % below
+// 9e-15, largest 4e-13 (symmetricEigen3 9e-17, 7e-13, 1e-12); with eigenvalues
+// 1e-5 apart both reach 1e-12.
 __device__ inline void strainFrame64(const double *m, double *vec, double *val) {
   const double s00 = m[0], s11 = m[4], s22 = m[8], s01 = m[3], s02 = m[6], s12 = m[7];
   auto expOf = [](double x) { return (int)(bitsOf(x) >> 52) & 0x7ff; };

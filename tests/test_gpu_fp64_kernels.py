@@ -192,4 +192,8 @@ def test_limiter_in_one_pass(gpu_lib, mesh, reconst, flow):
     top = np.abs(b).max(axis=(0, 2))
     if reconst == cases.RECONST_BJ:
         top[1:4] = top[1:4].max()  # the frame mixes the components
-    assert (np.abs(a - b).max(axis=(0, 2)) <= 1e-10 * top).all(), (np.abs(a - b).max(axis=(0, 2)), top)
+    # a uniform variable's gradient is the rounding of its values over the spacing
+    # (the pressure's, of the total energy it is recovered from)
+    prim = np.abs(np.stack([rho, u[:, 0], u[:, 1], u[:, 2], c.cv0[:, 4]], axis=1)).max(axis=0)
+    floor = 1e-14 * prim / gpu.Setup(c).vol.min() ** (1 / 3)
+    assert (np.abs(a - b).max(axis=(0, 2)) <= 1e-10 * top + floor).all(), (np.abs(a - b).max(axis=(0, 2)), top)
