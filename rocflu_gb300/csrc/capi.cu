@@ -1321,6 +1321,8 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   std::vector<int> bcell(nb), bpatch(nb);
   std::vector<double> bnx(nb), bny(nb), bnz(nb), bnm(nb), bd(3 * (size_t)nb);
   std::vector<int> pType(std::max(np, 1)), pOut(std::max(np, 1)), pOrder(std::max(np, 1));
+  std::vector<int> pOff(np + 1, 0);
+  for (int ip = 0; ip < np; ++ip) pOff[ip + 1] = g->patchFaceOff[ip + 1];
   std::vector<double> pK((size_t)kPatchK * std::max(np, 1), 0.0);
   for (int ip = 0; ip < np; ++ip) {
     pType[ip] = g->patchBcType[ip];
@@ -1478,6 +1480,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   PUT(V.bnx, bnx, R); PUT(V.bny, bny, R); PUT(V.bnz, bnz, R); PUT(V.bnm, bnm, R);
   PUT(V.bd, bd, R);
   PUT(V.patchType, pType, int); PUT(V.patchOutflow, pOut, int); PUT(V.patchOrder, pOrder, int);
+  PUT(V.patchOff, pOff, int);
   PUT(V.patchK, pK, double);
   PUT(V.cfOff, cfOff, int); PUT(V.cfEnt, cfEnt, int);
   PUT(V.stOff, stOff, int); PUT(V.stIdx, stIdx, int);

@@ -107,6 +107,7 @@ struct View {
   const R *bnx, *bny, *bnz, *bnm;
   const R *bd;                      // (3, nb): fc - cofg(cell)
   const int *patchType, *patchOutflow, *patchOrder;  // patchOutflow: the BCOPT type switch
+  const int *patchOff;              // each patch's first boundary face, and nb
   const double *patchK;             // kPatchK constants per patch (physics.cuh)
   // constrained gradients (CRECONSTC 1, constr.h): per cell its slot or -1
   // (null: none), per slot the constraint-row counts of the five variables
