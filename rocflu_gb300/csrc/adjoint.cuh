@@ -913,7 +913,7 @@ __global__ void __launch_bounds__(kBlock) kAdjGradFwd(View<R> V, AdjWork<R> W, c
       // records (a boundary face's or a missing one's is the cell's own, which
       // is no extreme), instead of one face's three dependent loads after
       // another's (with kAdjCell2's counted loop and kPatchSeed's own faces only,
-      // 4 unrolled steps of 32,768 cells with their gradient 2.31 -> 2.27 ms)
+      // 4 unrolled steps of 32,768 cells with their gradient 2.33 -> 2.28 ms)
       int codes[kMaxCellFaces], nbs[kMaxCellFaces];
 #pragma unroll
       for (int m = 0; m < kMaxCellFaces; ++m) codes[m] = cb + m < ce ? V.cfEnt[cb + m] : INT_MIN;
@@ -946,7 +946,6 @@ __global__ void __launch_bounds__(kBlock) kAdjGradFwd(View<R> V, AdjWork<R> W, c
       }
     }
     const R epsq = V.epsq[i];
-#pragma unroll 2
     for (int e = cb; e < ce; ++e) {
       const int code = V.cfEnt[e];
       R d[3];
