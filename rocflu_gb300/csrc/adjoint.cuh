@@ -1199,7 +1199,7 @@ __global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int 
           dl[k] = side ? D8(V.dv[k * n + c1]) : D8::seed(V.dv[k * n + c1], 5 + k);
           dr[k] = side ? D8::seed(V.dv[k * n + c2], 5 + k) : D8(V.dv[k * n + c2]);
         }
-        riemann1(P, cl, dl, cr, dr, D8((double)nx), D8((double)ny), D8((double)nz), D8((double)nm), flx);
+        riemann1(P, cl, dl, cr, dr, nx, ny, nz, nm, flx);
         contract(flx, fb, o8);
 #pragma unroll
         for (int m = 0; m < 8; ++m) out[8 * side + m] = (R)o8[m];
@@ -1233,7 +1233,7 @@ __global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int 
         ia = side ? D6(irl) : D6::seed(irl, 5);
         ib = side ? D6::seed(irr, 5) : D6(irr);
         if constexpr (kFlux == 0) {
-          riemann2(P, D6(nx), D6(ny), D6(nz), D6(nm), a, ia, b, ib, flx);
+          riemann2(P, nx, ny, nz, nm, a, ia, b, ib, flx);
           contract(flx, fbar, out + 6 * side);
         }
       }
@@ -1265,8 +1265,7 @@ __global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int 
         cr[0] = cl[0];
         reflect3(Q, cl + 1, cr + 1);
         cr[4] = cl[4];
-        riemann1(P, cl, dl, cr, dl, D8((double)V.bnx[b]), D8((double)V.bny[b]), D8((double)V.bnz[b]),
-                 D8((double)V.bnm[b]), flx);
+        riemann1(P, cl, dl, cr, dl, V.bnx[b], V.bny[b], V.bnz[b], V.bnm[b], flx);
         contract(flx, fb, o8);
 #pragma unroll
         for (int m = 0; m < 8; ++m) out[m] = (R)o8[m];
@@ -1282,7 +1281,7 @@ __global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int 
         r[0] = a[0];
         reflect3(Q, a + 1, r + 1);
         r[4] = a[4];
-        riemann2(P, D6(V.bnx[b]), D6(V.bny[b]), D6(V.bnz[b]), D6(V.bnm[b]), a, ia, r, ia, flx);
+        riemann2(P, V.bnx[b], V.bny[b], V.bnz[b], V.bnm[b], a, ia, r, ia, flx);
         contract(flx, fbar, out);
       }
       return;

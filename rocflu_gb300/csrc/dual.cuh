@@ -78,6 +78,52 @@ RFLU_DUAL_BINOP(-, a.d[k] - b.d[k])
 RFLU_DUAL_BINOP(*, a.d[k] * b.v + a.v * b.d[k])
 #undef RFLU_DUAL_BINOP
 
+// With a number that carries no derivative (a geometric factor, a parameter of
+// the gas): the products with its zero derivatives are not formed.
+template <typename D> struct Same { using type = D; };
+template <int N, typename T>
+__host__ __device__ inline Dual<N, T> operator*(const Dual<N, T> &a, const typename Same<T>::type &b) {
+  Dual<N, T> r;
+  r.v = a.v * b;
+#pragma unroll
+  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * b;
+  return r;
+}
+template <int N, typename T>
+__host__ __device__ inline Dual<N, T> operator*(const typename Same<T>::type &a, const Dual<N, T> &b) { return b * a; }
+template <int N, typename T>
+__host__ __device__ inline Dual<N, T> operator+(const Dual<N, T> &a, const typename Same<T>::type &b) {
+  Dual<N, T> r = a;
+  r.v = a.v + b;
+  return r;
+}
+template <int N, typename T>
+__host__ __device__ inline Dual<N, T> operator+(const typename Same<T>::type &a, const Dual<N, T> &b) { return b + a; }
+template <int N, typename T>
+__host__ __device__ inline Dual<N, T> operator-(const Dual<N, T> &a, const typename Same<T>::type &b) {
+  Dual<N, T> r = a;
+  r.v = a.v - b;
+  return r;
+}
+template <int N, typename T>
+__host__ __device__ inline Dual<N, T> operator-(const typename Same<T>::type &a, const Dual<N, T> &b) {
+  Dual<N, T> r;
+  r.v = a - b.v;
+#pragma unroll
+  for (int k = 0; k < N; ++k) r.d[k] = -b.d[k];
+  return r;
+}
+template <int N, typename T>
+__host__ __device__ inline Dual<N, T> operator/(const typename Same<T>::type &a, const Dual<N, T> &b) {
+  Dual<N, T> r;
+  const T ib = div_(T(1), b.v);
+  r.v = div_(a, b.v);
+  const T s = -(r.v * ib);
+#pragma unroll
+  for (int k = 0; k < N; ++k) r.d[k] = s * b.d[k];
+  return r;
+}
+
 template <int N, typename T>
 __host__ __device__ inline Dual<N, T> operator/(const Dual<N, T> &a, const Dual<N, T> &b) {
   Dual<N, T> r;
@@ -123,7 +169,7 @@ __host__ __device__ inline Dual<N, T> powConstExp(const Dual<N, T> &a, const Dua
 }
 template <int N, typename T>
 __host__ __device__ inline Dual<N, T> fabs_(const Dual<N, T> &a) {
-  return (a.v < T(0)) ? -a : a;
+  return neg_(a.v) ? -a : a;
 }
 template <int N, typename T>
 __host__ __device__ inline Dual<N, T> copysign_(const Dual<N, T> &a, const Dual<N, T> &b) {

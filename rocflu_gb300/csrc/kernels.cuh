@@ -96,8 +96,10 @@ constexpr bool kFixedSums = true;
 #else
 constexpr bool kFixedSums = false;
 #endif
+template <typename S> struct IsFp64 { static constexpr bool v = std::is_same<S, double>::value; };
+template <int N> struct IsFp64<Dual<N, double>> { static constexpr bool v = true; };
 template <typename S>
-constexpr bool shortFlux() { return kFixedSums && std::is_same<S, double>::value; }
+constexpr bool shortFlux() { return kFixedSums && IsFp64<S>::v; }
 
 // Reference arithmetic (the FP64 modes) reproduces the cons -> prim -> cons
 // round trip of CellGradientsMP on the fly; the mixed mode uses the
@@ -2658,8 +2660,8 @@ __global__ void __launch_bounds__(kBlock) kCellDtTile(View<R> V) {
 // plus grad . (fc - cofg).
 // ---------------------------------------------------------------------------
 template <typename R, typename L>
-__device__ inline void faceState(const View<R> &V, const L &ld, int c, typename L::S dx, typename L::S dy,
-                                 typename L::S dz, typename L::S *s, typename L::S &irCell) {
+__device__ inline void faceState(const View<R> &V, const L &ld, int c, R dx, R dy, R dz, typename L::S *s,
+                                 typename L::S &irCell) {
   using S = typename L::S;
   S q[5], gr[15];
   ld.prim5(c, q);
@@ -2686,20 +2688,21 @@ __device__ inline void faceState(const View<R> &V, const L &ld, int c, typename 
 template <typename S> __device__ inline S prm(double d, float) { return S(d); }
 template <> __device__ inline float prm<float>(double, float f) { return f; }
 
-template <typename S>
-__device__ inline void riemann2(const Params &P, S nx, S ny, S nz, S nm, const S *L, S irl, const S *Rt, S irr, S *flx) {
+template <typename S, typename T>
+__device__ inline void riemann2(const Params &P, T nx, T ny, T nz, T nm, const S *L, S irl, const S *Rt, S irr, S *flx) {
   if constexpr (shortFlux<S>()) {
-    const double g = P.refGamma, il = div_(1.0, L[0]), ir = div_(1.0, Rt[0]);
-    const double tl = L[4] * il, tr = Rt[4] * ir;  // p / rho
-    const double kl = 0.5 * (L[1] * L[1] + L[2] * L[2] + L[3] * L[3]);
-    const double kr = 0.5 * (Rt[1] * Rt[1] + Rt[2] * Rt[2] + Rt[3] * Rt[3]);
+    const double g = P.refGamma;
+    const S il = div_(1.0, L[0]), ir = div_(1.0, Rt[0]);
+    const S tl = L[4] * il, tr = Rt[4] * ir;  // p / rho
+    const S kl = 0.5 * (L[1] * L[1] + L[2] * L[2] + L[3] * L[3]);
+    const S kr = 0.5 * (Rt[1] * Rt[1] + Rt[2] * Rt[2] + Rt[3] * Rt[3]);
     if (P.spaceDiscr == 3) {
-      const double el = tl * P.refIg1 + kl, er = tr * P.refIg1 + kr;
+      const S el = tl * P.refIg1 + kl, er = tr * P.refIg1 + kr;
       hllcFluxShort(P.refG1, nx, ny, nz, nm, L[0], L[1], L[2], L[3], L[4], el, sqrt_(g * tl), el + irl * L[4], il,
                     Rt[0], Rt[1], Rt[2], Rt[3], Rt[4], er, sqrt_(g * tr), er + irr * Rt[4], flx);
       return;
     }
-    const double Hl = P.refKh * tl + kl, Hr = P.refKh * tr + kr;
+    const S Hl = P.refKh * tl + kl, Hr = P.refKh * tr + kr;
     if (P.spaceDiscr == 1)
       roeFluxShort(P.refG1, P.epsEntr, P.dissFact, nx, ny, nz, nm, L[0], L[1], L[2], L[3], L[4], Hl, Rt[0], Rt[1],
                    Rt[2], Rt[3], Rt[4], Hr, flx);
@@ -2713,38 +2716,38 @@ __device__ inline void riemann2(const Params &P, S nx, S ny, S nz, S nm, const S
     S gc = cp - div_(cp, g);
     S tl = div_(L[4], L[0] * gc), tr = div_(Rt[4], Rt[0] * gc);
     S Hl = perfHo(cp, tl, L[1], L[2], L[3]), Hr = perfHo(cp, tr, Rt[1], Rt[2], Rt[3]);
-    roeFlux(g, prm<S>(P.epsEntr, P.epsEntrF), prm<S>(P.dissFact, P.dissFactF), nx, ny, nz, nm, L[0], L[1], L[2], L[3],
+    roeFlux(g, prm<S>(P.epsEntr, P.epsEntrF), prm<S>(P.dissFact, P.dissFactF), S(nx), S(ny), S(nz), S(nm), L[0], L[1], L[2], L[3],
             L[4], Hl, Rt[0], Rt[1], Rt[2], Rt[3], Rt[4], Hr, flx);
   } else if (P.spaceDiscr == 3) {
     S el = perfEo(L[0], g, L[4], L[1], L[2], L[3]), al = sqrt_(div_(g * L[4], L[0]));
     S er = perfEo(Rt[0], g, Rt[4], Rt[1], Rt[2], Rt[3]), ar = sqrt_(div_(g * Rt[4], Rt[0]));
     S Hl = el + irl * L[4], Hr = er + irr * Rt[4];
-    hllcFlux(g, nx, ny, nz, nm, L[0], L[1], L[2], L[3], L[4], el, al, Hl, Rt[0], Rt[1], Rt[2], Rt[3], Rt[4], er, ar,
+    hllcFlux(g, S(nx), S(ny), S(nz), S(nm), L[0], L[1], L[2], L[3], L[4], el, al, Hl, Rt[0], Rt[1], Rt[2], Rt[3], Rt[4], er, ar,
              Hr, flx);
   } else {
     S gc = cp - div_(cp, g);
     S tl = div_(L[4], L[0] * gc), tr = div_(Rt[4], Rt[0] * gc);
     S al = sqrt_(g * gc * tl), ar = sqrt_(g * gc * tr);
     S Hl = perfHo(cp, tl, L[1], L[2], L[3]), Hr = perfHo(cp, tr, Rt[1], Rt[2], Rt[3]);
-    ausmFlux(nx, ny, nz, nm, L[0], L[1], L[2], L[3], L[4], Hl, al, Rt[0], Rt[1], Rt[2], Rt[3], Rt[4], Hr, ar, flx);
+    ausmFlux(S(nx), S(ny), S(nz), S(nm), L[0], L[1], L[2], L[3], L[4], Hl, al, Rt[0], Rt[1], Rt[2], Rt[3], Rt[4], Hr, ar, flx);
   }
 }
 
 // First-order interior flux from cv and dv (type H: FP64 in every mode).
 template <typename H>
-__device__ inline void riemann1(const Params &P, const H *cl, const H *dvl, const H *cr, const H *dvr, H nx, H ny,
-                                H nz, H nm, H *flx) {
+__device__ inline void riemann1(const Params &P, const H *cl, const H *dvl, const H *cr, const H *dvr, double nx,
+                                double ny, double nz, double nm, H *flx) {
   H rl = cl[0], irl = div_(H(1), rl), ul = cl[1] * irl, vl = cl[2] * irl, wl = cl[3] * irl;
   H rr = cr[0], irr = div_(H(1), rr), ur = cr[1] * irr, vr = cr[2] * irr, wr = cr[3] * irr;
   H pl = dvl[0], pr = dvr[0];
   if constexpr (shortFlux<H>()) {
     if (P.spaceDiscr == 1) {
       roeFluxShort(P.refG1, P.epsEntr, P.dissFact, nx, ny, nz, nm, rl, ul, vl, wl, pl,
-                   perfHo(P.refCp, dvl[1], ul, vl, wl), rr, ur, vr, wr, pr, perfHo(P.refCp, dvr[1], ur, vr, wr), flx);
+                   perfHo(H(P.refCp), dvl[1], ul, vl, wl), rr, ur, vr, wr, pr, perfHo(H(P.refCp), dvr[1], ur, vr, wr), flx);
       return;
     }
-    const double el = cl[4] * irl, er = cr[4] * irr;
-    const double Hl = el + irl * pl, Hr = er + irr * pr;
+    const H el = cl[4] * irl, er = cr[4] * irr;
+    const H Hl = el + irl * pl, Hr = er + irr * pr;
     if (P.spaceDiscr == 3)
       hllcFluxShort(P.refG1, nx, ny, nz, nm, rl, ul, vl, wl, pl, el, dvl[2], Hl, irl, rr, ur, vr, wr, pr, er, dvr[2],
                     Hr, flx);
@@ -2755,14 +2758,14 @@ __device__ inline void riemann1(const Params &P, const H *cl, const H *dvl, cons
   const H cp = H(P.refCp), g = H(P.refGamma);
   if (P.spaceDiscr == 1) {
     H Hl = perfHo(cp, dvl[1], ul, vl, wl), Hr = perfHo(cp, dvr[1], ur, vr, wr);
-    roeFlux(g, H(P.epsEntr), H(P.dissFact), nx, ny, nz, nm, rl, ul, vl, wl, pl, Hl, rr, ur, vr, wr, pr, Hr, flx);
+    roeFlux(g, H(P.epsEntr), H(P.dissFact), H(nx), H(ny), H(nz), H(nm), rl, ul, vl, wl, pl, Hl, rr, ur, vr, wr, pr, Hr, flx);
   } else if (P.spaceDiscr == 3) {
     H el = cl[4] * irl, er = cr[4] * irr;
     H Hl = el + irl * pl, Hr = er + irr * pr;
-    hllcFlux(g, nx, ny, nz, nm, rl, ul, vl, wl, pl, el, dvl[2], Hl, rr, ur, vr, wr, pr, er, dvr[2], Hr, flx);
+    hllcFlux(g, H(nx), H(ny), H(nz), H(nm), rl, ul, vl, wl, pl, el, dvl[2], Hl, rr, ur, vr, wr, pr, er, dvr[2], Hr, flx);
   } else {
     H Hl = cl[4] * irl + div_(pl, rl), Hr = cr[4] * irr + div_(pr, rr);
-    ausmFlux(nx, ny, nz, nm, rl, ul, vl, wl, pl, Hl, dvl[2], rr, ur, vr, wr, pr, Hr, dvr[2], flx);
+    ausmFlux(H(nx), H(ny), H(nz), H(nm), rl, ul, vl, wl, pl, Hl, dvl[2], rr, ur, vr, wr, pr, Hr, dvr[2], flx);
   }
 }
 
@@ -2873,7 +2876,7 @@ __device__ inline void faceFluxEval(const View<R> &V, const L &ld, int t, typena
       for (int k = 0; k < 5; ++k) { cl[k] = ld.cv(k, c1); cr[k] = ld.cv(k, c2); }
 #pragma unroll
       for (int k = 0; k < 3; ++k) { dl[k] = ld.dv(k, c1); dr[k] = ld.dv(k, c2); }
-      riemann1(P, cl, dl, cr, dr, H((double)nx), H((double)ny), H((double)nz), H((double)nm), fd);
+      riemann1(P, cl, dl, cr, dr, nx, ny, nz, nm, fd);
 #pragma unroll
       for (int k = 0; k < 5; ++k) flx[k] = cvt<S>(fd[k]);
     } else {
@@ -2881,9 +2884,9 @@ __device__ inline void faceFluxEval(const View<R> &V, const L &ld, int t, typena
       R dl[3], dr[3];
       faceOffset(V, f, 0, dl);
       faceOffset(V, f, 1, dr);
-      faceState(V, ld, c1, S(dl[0]), S(dl[1]), S(dl[2]), Lf, irl);
-      faceState(V, ld, c2, S(dr[0]), S(dr[1]), S(dr[2]), Rt, irr);
-      riemann2(P, S(nx), S(ny), S(nz), S(nm), Lf, irl, Rt, irr, flx);
+      faceState(V, ld, c1, dl[0], dl[1], dl[2], Lf, irl);
+      faceState(V, ld, c2, dr[0], dr[1], dr[2], Rt, irr);
+      riemann2(P, nx, ny, nz, nm, Lf, irl, Rt, irr, flx);
     }
   } else {
     const int b = t - V.nf, c = V.bcell[b], ip = V.bpatch[b];
@@ -2902,18 +2905,17 @@ __device__ inline void faceFluxEval(const View<R> &V, const L &ld, int t, typena
         cr[0] = cl[0];
         reflect3(Q, cl + 1, cr + 1);
         cr[4] = cl[4];
-        riemann1(P, cl, dl, cr, dl, H((double)V.bnx[b]), H((double)V.bny[b]), H((double)V.bnz[b]),
-                 H((double)V.bnm[b]), fd);
+        riemann1(P, cl, dl, cr, dl, V.bnx[b], V.bny[b], V.bnz[b], V.bnm[b], fd);
 #pragma unroll
         for (int k = 0; k < 5; ++k) flx[k] = cvt<S>(fd[k]);
       } else {
         const size_t nb = V.nb;
         S Lf[5], Rt[5], irl;
-        faceState(V, ld, c, S(V.bd[b]), S(V.bd[nb + b]), S(V.bd[2 * nb + b]), Lf, irl);
+        faceState(V, ld, c, V.bd[b], V.bd[nb + b], V.bd[2 * nb + b], Lf, irl);
         Rt[0] = Lf[0];
         reflect3(Q, Lf + 1, Rt + 1);
         Rt[4] = Lf[4];
-        riemann2(P, S(V.bnx[b]), S(V.bny[b]), S(V.bnz[b]), S(V.bnm[b]), Lf, irl, Rt, irl, flx);
+        riemann2(P, V.bnx[b], V.bny[b], V.bnz[b], V.bnm[b], Lf, irl, Rt, irl, flx);
       }
       return;
     }
@@ -2928,7 +2930,7 @@ __device__ inline void faceFluxEval(const View<R> &V, const L &ld, int t, typena
     } else {
       const size_t nb = V.nb;
       S Lf[5], irl;
-      faceState(V, ld, c, S(V.bd[b]), S(V.bd[nb + b]), S(V.bd[2 * nb + b]), Lf, irl);
+      faceState(V, ld, c, V.bd[b], V.bd[nb + b], V.bd[2 * nb + b], Lf, irl);
       patch2(P, type, V.patchOutflow[ip], V.patchK + kPatchK * ip, Lf, S(V.bnx[b]), S(V.bny[b]), S(V.bnz[b]),
              S(V.bnm[b]), flx);
     }

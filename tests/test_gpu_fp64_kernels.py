@@ -152,6 +152,31 @@ def test_short_fluxes(gpu_lib, order, discr, mach):
     assert (np.abs(a - b) / np.abs(b).max(axis=0)).max() < 1e-12
 
 
+@pytest.mark.parametrize("mesh", ["hex", "symmetry"])
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("discr", [cases.DISCR_ROE, cases.DISCR_HLLC, cases.DISCR_AUSM])
+@pytest.mark.parametrize("mach", [0.4, -2.5])
+def test_short_flux_derivatives(gpu_lib, mesh, order, discr, mach):
+    """Tangent and adjoint through the fp64 mode's fluxes (dual numbers over
+    the short form, normals without derivatives) against the FP64_EXACT ones,
+    unlimited gradients: 1e-11 of the largest value, some 500 roundings with
+    room for their cancellation."""
+    num = cases.Numerics(space_order=order, space_discr=discr, reconst=0, cfl=0.4)
+    c = cases.mirror_box(5, axes=(0, 1, 2), num=num) if mesh == "symmetry" else cases.blast_hex(6, num=num)
+    for p in c.patches:
+        p.order = order
+    rng = np.random.default_rng(9)
+    n = len(c.cv0)
+    rho, p = 1.0 + 0.2 * rng.random(n), 1.0 + 0.2 * rng.random(n)
+    u = (mach * np.sqrt(1.4) + 0.05 * rng.standard_normal(n), 0.05 * rng.standard_normal(n), 0.05 * rng.standard_normal(n))
+    c.cv0 = cases.conserved(rho, *u, p, c.num.gamma)
+    dot, bar = rng.standard_normal(c.cv0.shape), rng.standard_normal(c.cv0.shape)
+    a, b = gpu.Region(c, "fp64"), gpu.Region(c, "fp64_exact")
+    for x, y in ((a.jvp(c.cv0, dot), b.jvp(c.cv0, dot)), (a.vjp(c.cv0, bar), b.vjp(c.cv0, bar))):
+        assert np.isfinite(y).all()
+        assert np.abs(x - y).max() <= 1e-11 * np.abs(y).max()
+
+
 @pytest.mark.parametrize("mesh", ["hex", "tets", "symmetry", "periodic"])
 @pytest.mark.parametrize("reconst", [cases.RECONST_BJ, cases.RECONST_BJ_COMP])
 @pytest.mark.parametrize("flow", ["wavy", "shear", "still", "steep", "small"])
