@@ -458,8 +458,20 @@ __global__ void __launch_bounds__(kBlock) kTanWeno(View<R> V, AdjWork<R> W) {
   storeGrad(V, i, gv);
 }
 
+// The face kernels of the derivatives in FP64 hold 160 to 216 registers, so a
+// block of 256 threads was alone on its SM (8 warps, the FP64 pipe 66 to 75 %
+// busy): three blocks of 128 are 12 warps.  196,608 tetrahedra, Roe: kTanFlux
+// 405 -> 314 us, kAdjFace 327 -> 275 us (FP64 pipe 82 and 85 % busy).
+template <typename R> constexpr int kFaceBlock = Layout<R>::packed ? kBlock : 128;
+template <typename R> constexpr int kFaceBlocks = Layout<R>::packed ? 1 : 3;
 template <typename R>
-__global__ void __launch_bounds__(kBlock) kTanFlux(View<R> V, AdjWork<R> W) {
+inline Shape faceShape(const View<R> &V, long long n) {
+  const int b = std::min(kFaceBlock<R>, shapeFor(V, n).block);
+  return {(int)((n + b - 1) / b), b};
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kFaceBlock<R>, kFaceBlocks<R>) kTanFlux(View<R> V, AdjWork<R> W) {
   gridOrder();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int nT = V.nf + V.nb;
@@ -1164,7 +1176,7 @@ __device__ inline void contract(const Dual<N, T> *flx, const T *fbar, T *out) {
 // for HLLC, mixed mode, 95,232 faces: 12 stage adjoints of an
 // unrolled gradient 2.85 -> 2.53 ms.
 template <typename R, int kFlux>
-__global__ void __launch_bounds__(kBlock) kAdjFace(View<R> V, AdjWork<R> W, int t0, int t1) {
+__global__ void __launch_bounds__(kFaceBlock<R>, kFlux ? kFaceBlocks<R> : 1) kAdjFace(View<R> V, AdjWork<R> W, int t0, int t1) {
   gridOrder();
   const int t = t0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= t1) return;
@@ -2074,7 +2086,7 @@ struct AdjointOps {
       launchOrdered(kTanGrad<R>, shapeFor(V, V.nc), s, V, W, haveG);
     }
     if (isWeno(V.p)) launchOrdered(kTanWeno<R>, shapeFor(V, V.nc), s, V, W);
-    launchOrdered(kTanFlux<R>, shapeFor(V, (long long)nT), s, V, W);
+    launchOrdered(kTanFlux<R>, faceShape(V, nT), s, V, W);
     launchOrdered(kTanGather<R>, shapeFor(V, V.nc), s, V, W, rhsDotRef);
   }
   static void gradFwd(const View<R> &V, const AdjWork<R> &W, const double *lamRef, cudaStream_t s) {
@@ -2098,9 +2110,9 @@ struct AdjointOps {
   }
   static void interiorFaces(const View<R> &V, const AdjWork<R> &W, cudaStream_t s) {
     const int flux = V.p.spaceOrder > 1 ? V.p.spaceDiscr : 0;
-    if (flux == 1) launchOrdered(kAdjFace<R, 1>, shapeFor(V, (long long)V.nf), s, V, W, 0, V.nf);
-    else if (flux == 3) launchOrdered(kAdjFace<R, 3>, shapeFor(V, (long long)V.nf), s, V, W, 0, V.nf);
-    else launchOrdered(kAdjFace<R, 0>, shapeFor(V, (long long)V.nf), s, V, W, 0, V.nf);
+    if (flux == 1) launchOrdered(kAdjFace<R, 1>, faceShape(V, V.nf), s, V, W, 0, V.nf);
+    else if (flux == 3) launchOrdered(kAdjFace<R, 3>, faceShape(V, V.nf), s, V, W, 0, V.nf);
+    else launchOrdered(kAdjFace<R, 0>, faceShape(V, V.nf), s, V, W, 0, V.nf);
   }
   // The boundary faces' kernel (dual numbers through the patch fluxes; few
   // faces, a small grid) runs on a second stream beside the interior faces'
@@ -2111,13 +2123,13 @@ struct AdjointOps {
     const int nT = V.nf + V.nb;
     if (V.nf == 0 || V.nb == 0) {
       if (V.nb == 0 && nT > 0) interiorFaces(V, W, s);
-      else if (nT > 0) launchOrdered(kAdjFace<R, 0>, shapeFor(V, (long long)nT), s, V, W, 0, nT);
+      else if (nT > 0) launchOrdered(kAdjFace<R, 0>, faceShape(V, nT), s, V, W, 0, nT);
       return;
     }
     SideStream &ss = sideStream();
     cudaEventRecord(ss.fork, s);
     cudaStreamWaitEvent(ss.stream, ss.fork, 0);
-    const Shape sh = shapeFor(V, (long long)V.nb);  // after an event: launched plainly
+    const Shape sh = faceShape(V, V.nb);  // after an event: launched plainly
     kAdjFace<R, 0><<<sh.grid, sh.block, 0, ss.stream>>>(V, W, V.nf, nT);
     cudaEventRecord(ss.join, ss.stream);
     interiorFaces(V, W, s);
