@@ -2983,13 +2983,13 @@ __device__ inline void gatherRhs(const View<R> &V, const T *flux, int i, T *rhs)
       const int f = code >> 1;
       T fl[5];
       loadFlux<R>(flux, nT, f, fl);
-      if (code & 1) {
+      // the side's sign as a factor: the same sums, and lanes on either side of
+      // their faces add together (as two branches, the FP64 pipe ran both;
+      // with afterUpdate's skip, 40 first-order steps of 6,400 cells 3.04 ->
+      // 2.85 ms, 2 steps of 421,875 hexahedra 6.09 -> 5.87 ms)
+      const T sg = (code & 1) ? T(-1) : T(1);
 #pragma unroll
-        for (int k = 0; k < 5; ++k) rhs[k] = rhs[k] - fl[k];
-      } else {
-#pragma unroll
-        for (int k = 0; k < 5; ++k) rhs[k] = rhs[k] + fl[k];
-      }
+      for (int k = 0; k < 5; ++k) rhs[k] = fma(fl[k], sg, rhs[k]);
     } else {
       const int b = -code - 1;
       const int k0 = patchLeavesDensity(V.patchType[V.bpatch[b]]) ? 1 : 0;  // walls leave rhs(DENS)
@@ -3044,7 +3044,15 @@ __device__ inline void afterUpdate(const View<R> &V, int i, double *cv, double &
     }
   }
   const double gamma = P.gRT;
-  {
+  // The pressure of the bounds check is formed from the velocities instead of
+  // the momenta; it is positive wherever pr is so by far more than the rounding
+  // of the total energy (2^-36 of it against some 2^-49, squares in range), and
+  // only other cells form it.
+  auto expo = [](double x) { return (int)(bitsOf(x) >> 52); };  // of a positive number
+  const int ep = expo(pr), ee = expo(cv[4]), er = expo(cv[0]);
+  const bool clear = ep < 0x7ff && ep + 36 >= ee && abs(ee - 1023) <= 100 && abs(er - 1023) <= 100 &&
+                     expo(gamma) <= 1023 + 3;
+  if (!clear) {
     double r = cv[0], ir = div_(1.0, r);
     double u = ir * cv[1], v = ir * cv[2], w = ir * cv[3];
     double Eo = ir * cv[4];

@@ -222,3 +222,28 @@ def test_limiter_in_one_pass(gpu_lib, mesh, reconst, flow):
     prim = np.abs(np.stack([rho, u[:, 0], u[:, 1], u[:, 2], c.cv0[:, 4]], axis=1)).max(axis=0)
     floor = 1e-14 * prim / gpu.Setup(c).vol.min() ** (1 / 3)
     assert (np.abs(a - b).max(axis=(0, 2)) <= 1e-10 * top + floor).all(), (np.abs(a - b).max(axis=(0, 2)), top)
+
+
+@pytest.mark.parametrize("rho0", [1.0, 1e-35])
+@pytest.mark.parametrize("p0", [1e-12, 1e-2])
+@pytest.mark.parametrize("cfl", [1, 3])
+def test_bounds_check_only_near_zero(gpu_lib, rho0, p0, cfl):
+    """Still gas overdriven to pressures either side of zero, inside and
+    outside the 1e-12 of the bounds check and inside and outside the range in
+    which the update skips it: counters and bits of the oracle."""
+    c = cases.sod(40, 1, 1)
+    c.num.rk_scheme = cases.RK_EULER
+    rng = np.random.default_rng(4)
+    n = len(c.cv0)
+    p, rho, z = p0 * 2 * rng.random(n), rho0 * (1 + 0.5 * rng.random(n)), np.zeros(n)
+    c.cv0 = cases.conserved(rho, z, z, z, p, 1.4)
+    dt = cfl * 0.025 / np.sqrt(1.4 * p0 / rho0)
+    o = Oracle(c)
+    o.rk_stage(1, dt)
+    pf, neg, nan = o.counters()
+    assert nan == 0 and (pf > 0) == (cfl == 3) and (neg > 0) == (cfl == 3 and p0 == 1e-12)
+    r = gpu.Region(c, "fp64_exact")
+    r.rk_stage(1, dt)
+    st = r.status()
+    assert (st["posFixCells"], st["negPCells"], st["nanCells"]) == (pf, neg, nan)
+    np.testing.assert_array_equal(r.download()[0], o.state()[0])
