@@ -980,14 +980,12 @@ __device__ inline float tileDtSum(const View<float> &V, int i, const float *recs
   return sum;
 }
 
-// Eigenvalues (ascending) and eigenvectors (columns) of the strain rate in
 // FP32: cyclic Jacobi rotations as symmetricEigen3 takes them, each angle's
-// tangent as b / (d + sgn(d) sqrt(d^2 + b^2)), d = r_qq - r_pp, b = 2 r_pq (one
-// root, one reciprocal and one reciprocal root, about 40 instructions a
-// rotation instead of 60), until the off-diagonals are below 2^-25 of the
-// matrix, half a rounding of its FP32 entries; the general routine's 1e-12
-// costs a sweep more that turns the axes by less than that.  Measured with
-// every cell's frame active, 128^3: 10 steps 16.07 -> 15.74 ms.
+// tangent from one division and its cosine from one reciprocal root, to
+// off-diagonals of 3e-8: the start of strainFrame64's FP64 sweep.  The mixed
+// mode's own frame stays with symmetricEigen3: with these rotations 10 steps of
+// 2.1 M cells took 16.0 -> 15.7 ms but ended 8.8e-8 from the FP64 result
+// instead of 3.7e-8, at either tolerance.
 __device__ inline void jacobi3(float &r0, float &r1, float &r2, float r01, float r02, float r12, float *vec) {
   const float total = r0 * r0 + r1 * r1 + r2 * r2 + 2.f * (r01 * r01 + r02 * r02 + r12 * r12);
 #pragma unroll
@@ -1019,13 +1017,6 @@ __device__ inline void jacobi3(float &r0, float &r1, float &r2, float r01, float
     rotate(r0, r2, r02, r01, r12, vec, vec + 6);
     rotate(r1, r2, r12, r01, r02, vec + 3, vec + 6);
   }
-}
-__device__ inline void strainFrame(const float *m, float *vec, float *val) {
-  val[0] = m[0];
-  val[1] = m[4];
-  val[2] = m[8];
-  jacobi3(val[0], val[1], val[2], m[3], m[6], m[7], vec);
-  sortAxes(val, vec);
 }
 
 template <bool kDt, bool kTiled, int kRc>
@@ -1176,7 +1167,7 @@ __device__ inline float gradLimitPacked(const View<float> &V, int i, float *g, f
     for (int a = 0; a < 3; ++a)
 #pragma unroll
       for (int b = 0; b < 3; ++b) Sy[a + 3 * b] = 0.5f * (G[a + 3 * b] + G[b + 3 * a]);
-    strainFrame(Sy, A, ev);
+    symmetricEigen3(Sy, A, ev);
     float mx = fabsf(ev[0]);
     mx = fmax2(mx, fabsf(ev[1]));
     mx = fmax2(mx, fabsf(ev[2]));
