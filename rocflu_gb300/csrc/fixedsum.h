@@ -125,9 +125,15 @@ RFLU_HD inline double fixResult(const FixSum &a, int scale) {
 #endif
 }
 
+// The smallest exponent of a block's largest weight: below it the smallest
+// result (values of 2^-500) would leave the normal doubles.
+constexpr int kFixWeightEmin = 610;
+
 // |w| < 2^x for the largest magnitude of a block of weights: its biased
-// exponent minus 1022; kFixBadScale for what fixOf does not take (or none).
-RFLU_HD inline int fixScale(int eMax) { return (eMax == 0 || eMax == kFixBad) ? kFixBadScale : eMax - 1022; }
+// exponent minus 1022; kFixBadScale for what the sums do not take (or none).
+RFLU_HD inline int fixScale(int eMax) {
+  return (eMax < kFixWeightEmin || eMax == kFixBad) ? kFixBadScale : eMax - 1022;
+}
 // A weight of that block in units of 2^(x - 55), rounded to nearest.
 RFLU_HD inline int64_t fixWeight(double w, int eMax) {
   const FixNum f = fixOf(w);
