@@ -331,6 +331,7 @@ struct Ctx : CtxBase {
   bool constrBurning = false;    // a constrained gradient (CRECONSTC 1) holds a burning injection face's row (cpOff/cpEnt)
   double *work = nullptr;        // adjoint workspace (allocated by the first adjoint call)
   int tsWidthLazy = 0;           // ... and the width of its transposed-stencil weights
+  int stWidth = 0;               // most stencil members of a cell
   size_t workBytes = 0;
   // scratch state (allocated by the first call that needs it): master cv,
   // dependent variables, primitive records, RK accumulator and scalars of the
@@ -392,6 +393,31 @@ struct Ctx : CtxBase {
     return RFLU_OK;
   }
 
+  // The fixed-point sums' arrays (View::fxIdx) on the meshes that gain from
+  // them.  The sums' scratch (seven values per cell) is the face-flux array.
+  int planFixedSums() {
+    if (V.p.precision != RFLU_PREC_FP64 || V.p.spaceOrder < 2 || 5 * ((size_t)V.nf + V.nb) < 7 * (size_t)V.nc)
+      return RFLU_OK;
+    const size_t nc = V.nc;
+    if (stWidth < 1 || stWidth > kFixMaxTerms || !allocOptional(&V.fxScale, nc)) return RFLU_OK;
+    int slow = 0, *dev = reinterpret_cast<int *>(staging);
+    RFLU_CUDA(cudaMemsetAsync(dev, 0, sizeof(int), stream));
+    ops->fixedSetup(V, dev, stream);
+    RFLU_CUDA(cudaMemcpyAsync(&slow, dev, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    RFLU_CUDA(cudaStreamSynchronize(stream));
+    // Venkatakrishnan's limiter gains less from its own kernel: 131,712
+    // tetrahedra 322 us against 376 with no such warp, 333 against 308 with 39 %
+    constexpr double kFixVenkatShare = 0.25;
+    if (V.p.reconst == 11 && (long long)slow * 32 > kFixVenkatShare * V.nc) return RFLU_OK;
+    V.fxWidth = stWidth;
+    if (!allocOptional(&V.fxW, 3 * (size_t)stWidth * nc) || !allocOptional(&V.fxIdx, (size_t)stWidth * nc)) {
+      V.fxIdx = nullptr;
+      return RFLU_OK;
+    }
+    ops->fixedSetup(V, nullptr, stream);
+    RFLU_CUDA(cudaStreamSynchronize(stream));
+    return RFLU_OK;
+  }
   int create(const rflu_grid_desc *g, const rflu_num_desc *num);
   int patchConstants(const rflu_grid_desc *g, int ip, const rflu_num_desc *num, int *bcOpt, double *K);
   int buildTiles(const std::vector<int> &cfOff, const std::vector<int> &cfEnt, const std::vector<int> &stOff,
@@ -1451,6 +1477,8 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
       }
   }
 
+  for (int i = 0; i < nc; ++i) stWidth = std::max(stWidth, stOff[i + 1] - stOff[i]);
+
   // ---- device upload -----------------------------------------------------------
   V.nc = nc; V.nf = nf; V.nb = nb;
   RFLU_CUDA(cudaDeviceGetAttribute(&V.sms, cudaDevAttrMultiProcessorCount, device));
@@ -1508,17 +1536,6 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
     }
   } else {
     PUT(V.wx, wx, R); PUT(V.wy, wy, R); PUT(V.wz, wz, R);
-    // the fixed-point sums' weights (configure fills them); the sums' scratch
-    // (seven values per cell) is the face-flux array
-    int w = 0;
-    for (int i = 0; i < nc; ++i) w = std::max(w, stOff[i + 1] - stOff[i]);
-    if (num->precision == RFLU_PREC_FP64 && num->spaceOrder > 1 && w > 0 && w <= kFixMaxTerms &&
-        5 * ((size_t)nf + nb) >= 7 * (size_t)nc) {
-      V.fxWidth = w;
-      if (!allocOptional(&V.fxW, 3 * (size_t)w * nc) || !allocOptional(&V.fxScale, nc) ||
-          !allocOptional(&V.fxIdx, (size_t)w * nc))
-        V.fxIdx = nullptr;
-    }
   }
   // transposed stencil (adjoint of the LSQ gradient, every mode)
   PUT(V.tsOff, tsOff, int); PUT(V.tsCell, tsCell, int); PUT(V.tsEnt, tsEnt, int);
@@ -1654,6 +1671,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   workBytes = sizeof(R) * (size_t)(130 * (size_t)nc + 24 * ((size_t)nf + nb) + 64) + sizeof(int) * 10 * (size_t)nc + 256;
   ops->configure(V);
   RFLU_CUDA(cudaDeviceSynchronize());
+  if ((rc = planFixedSums())) return rc;
   V.tileGrid = ops->tileGrid(V, 0, &V.tileBufs);
   V.tileGridDt = ops->tileGrid(V, 1, &V.tileBufsDt);
   return checkLaunch("rflu_gpu_create");

@@ -138,7 +138,8 @@ struct View {
   // RFLU_PREC_FP64: the stencil entry-major (entry k of cell i at k*nc + i)
   // for the fixed-point sums (fixedsum.h): member (-1 past the end), the
   // weights' halves (component c at (c*fxWidth + k)*nc + i) in units of
-  // 2^(fxScale - 55); null: the FP64 sums
+  // 2^(e - 1077) with e the component's exponent in the cell's packed
+  // fxScale (fixCellWeights); null: the FP64 sums
   int *fxIdx;
   int2 *fxW;
   int *fxScale;

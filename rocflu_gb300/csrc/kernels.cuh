@@ -1437,13 +1437,22 @@ __device__ inline void cpAsync8(void *smemDst, const void *gSrc) {
 // the latency of the members' gathers at 12 warps per SM (168 registers).
 // Measured, 421,875 hexahedra of 26 members, FP64 pipe 100% busy before: about
 // 440 us of the gradient kernel -> 235 us in the three kernels below; 131,712
-// tetrahedra of 40: 260 -> 132 us.  The block whose largest
-// magnitude sets the unit is the cell's own stencil, per variable, so the
-// rounding is 2^-55 of the largest value the fit sees, below that of the FP64
-// differences and partial sums.  Cells the fixed point does not take
-// (values beyond 2^+-500, denormals, infinities, NaN, reflected members, more
-// than kFixMaxTerms members) run the FP64 loop.  FP64_EXACT keeps the FP64
-// loop for its bits, the mixed mode its FP32 sums.
+// tetrahedra of 40: 260 -> 132 us.  The block whose largest magnitude sets the
+// unit is, for the values, the cell's own stencil and variable, for the weights
+// its component.  The rounding, 2^-55 of the largest value the fit sees and
+// 2^-56 of the largest weight, is below that of the FP64 differences and partial
+// sums while the weights are of like size (fixCellWeights: cells up to about
+// twice as long as wide); the gradient of a cell is meant as a vector, a
+// component far smaller than the others is rounded at their size.  Cells the
+// fixed point does not take (weights of other sizes, values beyond 2^+-500,
+// denormals, infinities, NaN, reflected members, more than kFixMaxTerms members)
+// run the FP64 loop.  Gradient and limiter with none, half and all of the cells
+// so, against the kernels of one thread per cell or variable with all sums in
+// FP64: 421,875 hexahedra with Barth-Jespersen limiters 508, 600, 680 us against
+// 965, 959, 909; unlimited 237, 331, 423 against 695; WENO 935, 1012, 1090
+// against 1363; 131,712 tetrahedra with Venkatakrishnan's 322, 333, 408 against
+// 376, 308, 376 (kFixVenkatShare).  FP64_EXACT keeps the FP64 loop for its bits,
+// the mixed mode its FP32 sums.
 // ---------------------------------------------------------------------------
 constexpr int kFixBlock = 128;
 constexpr int kFixDepth = 8;  // members in flight per thread (a power of two)
@@ -1508,31 +1517,43 @@ __global__ void __launch_bounds__(kBlock) kFixExponents(View<R> V, FixFields F) 
   F.eMax[i] = w;
 }
 
-// The members and weights of View::fxIdx / fxW / fxScale from the stencil CSR
-// (once per context).
+// The exponents of each cell's weights (View::fxScale, fixCellWeights) and the
+// number of warps that hold a cell whose sums stay in FP64: its own weights say
+// so, or a member seen reflected.
+template <typename R>
+__global__ void __launch_bounds__(kBlock) kFixCells(View<R> V, int *slow) {
+  gridOrder();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  bool fp64 = false;
+  if (i < V.nc) {
+    const int sb = V.stOff[i], n = V.stOff[i + 1] - sb;
+    int packed = fixCellWeights(V.wx + sb, V.wy + sb, V.wz + sb, n);
+    if (V.stXf)
+      for (int s = sb; s < sb + n; ++s)
+        if (V.stXf[s] >= 0) packed = kFixNoWeights;
+    V.fxScale[i] = packed;
+    fp64 = packed == kFixNoWeights;
+  }
+  if (__any_sync(0xffffffffu, fp64) && (threadIdx.x & 31) == 0) atomicAdd(slow, 1);
+}
+
+// The members and weights of View::fxIdx / fxW from the stencil CSR (once per
+// context).
 template <typename R>
 __global__ void __launch_bounds__(kBlock) kFixWeights(View<R> V) {
   gridOrder();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const size_t n = V.nc;
-  const int sb = V.stOff[i], cnt = V.stOff[i + 1] - sb;
-  int eMax = 0;
-  bool ok = cnt <= kFixMaxTerms;
-  for (int s = sb; s < sb + cnt; ++s) {
-    eMax = max(eMax, max(fixOf((double)V.wx[s]).e, max(fixOf((double)V.wy[s]).e, fixOf((double)V.wz[s]).e)));
-    if (V.stXf && V.stXf[s] >= 0) ok = false;
-  }
-  const int scale = fixScale(eMax);
-  V.fxScale[i] = ok ? scale : kFixBadScale;
+  const int sb = V.stOff[i], cnt = V.stOff[i + 1] - sb, packed = V.fxScale[i];
   for (int k = 0; k < V.fxWidth; ++k) {
     const bool on = k < cnt;
     V.fxIdx[k * n + i] = on ? V.stIdx[sb + k] : -1;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       FixHalves h{0, 0};
-      if (on && ok && scale != kFixBadScale)
-        h = fixSplit(fixWeight((double)(c == 0 ? V.wx : c == 1 ? V.wy : V.wz)[sb + k], eMax));
+      if (on && packed != kFixNoWeights)
+        h = fixSplit(fixWeight((double)(c == 0 ? V.wx : c == 1 ? V.wy : V.wz)[sb + k], fixWeightExp(packed, c)));
       V.fxW[(c * (size_t)V.fxWidth + k) * n + i] = make_int2(h.hi, h.lo);
     }
   }
@@ -1554,9 +1575,9 @@ __global__ void __launch_bounds__(kFixBlock, 3) kGradFixed(View<R> V, const R *q
   unsigned emax[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) emax[v] = fixExpOf(ew, v);
-  const int scale = V.fxScale[i];
+  const int packed = V.fxScale[i];
   R g[15];
-  if (scale != kFixBadScale && max(max(max(emax[0], emax[1]), max(emax[2], emax[3])), emax[4]) != kFixExpBad) {
+  if (packed != kFixNoWeights && max(max(max(emax[0], emax[1]), max(emax[2], emax[3])), emax[4]) != kFixExpBad) {
     // a cell's five values in units of the stencil's exponents: the ten-bit
     // differences of all five come from one subtraction (no field borrows)
     auto load = [&](int j, long long *m, unsigned long long &e) {
@@ -1627,7 +1648,8 @@ __global__ void __launch_bounds__(kFixBlock, 3) kGradFixed(View<R> V, const R *q
       fetch(k + kFixDepth);  // into the slot just read
     }
 #pragma unroll
-    for (int k = 0; k < 15; ++k) g[k] = (R)fixResult(a[k], scale - 55 + (int)emax[k / 3] + kFixEmin - 1 - 1077);
+    for (int k = 0; k < 15; ++k)
+      g[k] = (R)fixResult(a[k], fixScale(fixWeightExp(packed, k % 3)) - 55 + (int)emax[k / 3] + kFixEmin - 1 - 1077);
   } else {
     R qi[5];
 #pragma unroll
@@ -3486,11 +3508,15 @@ struct Launch {
     }
     if (V.tsW) launchOrdered(kTsWeights<R>, shapeFor(V, V.nc), s, V);
   }
-  static void configure(const View<R> &V) {
+  // The set-up of the fixed-point sums: the cells (View::fxScale; *slow is
+  // added the warps with a cell in FP64), then, with fxIdx and fxW, the weights.
+  static void fixedSetup(const View<R> &V, int *slow, cudaStream_t s) {
     if constexpr (kFixedSums && !Layout<R>::packed) {
-      const Shape sh = shapeFor(V, V.nc);
-      if (V.fxIdx) kFixWeights<R><<<sh.grid, sh.block>>>(V);
+      if (slow) launchOrdered(kFixCells<R>, shapeFor(V, V.nc), s, V, slow);
+      else launchOrdered(kFixWeights<R>, shapeFor(V, V.nc), s, V);
     }
+  }
+  static void configure(const View<R> &V) {
     if (V.tiled) {
       setTileSmem<false, 0>(V); setTileSmem<false, 10>(V); setTileSmem<false, 100>(V); setTileSmem<false, 11>(V);
       setTileSmem<true, 0>(V); setTileSmem<true, 10>(V); setTileSmem<true, 100>(V); setTileSmem<true, 11>(V);

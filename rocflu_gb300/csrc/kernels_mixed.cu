@@ -29,7 +29,7 @@ cudaError_t mixedRefineCheck(long long n, unsigned long long seed, double *maxRe
 const Ops<float> *opsMixed() {
   using L = mixed::Launch<float>;
   static const Ops<float> ops = {L::initState, L::initFromRef, L::gradLimit, L::faceFlux,  L::gatherRhs, L::gatherUpdate,
-                                 L::timestep,  L::stepEnd,   L::stepStart, L::configure, L::tileGrid, mixed::AdjointOps<float>::jvp, mixed::AdjointOps<float>::vjp,
+                                 L::timestep,  L::stepEnd,   L::stepStart, L::configure, L::fixedSetup, L::tileGrid, mixed::AdjointOps<float>::jvp, mixed::AdjointOps<float>::vjp,
                                  mixed::AdjointOps<float>::patchPressure, L::adjointSetup,
                                  L::updateFromRhs, L::addRhs, mixed::AdjointOps<float>::limiterBranches};
   return &ops;

@@ -21,6 +21,8 @@ struct Ops {
   void (*stepEnd)(const View<R> &, cudaStream_t);
   void (*stepStart)(const View<R> &, cudaStream_t);  // dt reduction + first-stage gradients
   void (*configure)(const View<R> &);                  // mesh-dependent kernel attributes
+  // the fixed-point sums' cells (slow given) or weights (slow null)
+  void (*fixedSetup)(const View<R> &, int *slow, cudaStream_t);
   int (*tileGrid)(const View<R> &, int withDt, int *bufs);  // CTAs of the persistent tiled kernels, tile buffers per CTA
   // tangent / adjoint of the residual (FP64 modes only; null elsewhere)
   void (*jvp)(const View<R> &, const double *cvDot, double *rhsDot, double *work, cudaStream_t);
