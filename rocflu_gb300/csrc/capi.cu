@@ -21,6 +21,7 @@
 #include "convert.cuh"
 #include "constr.h"
 #include "ctx.h"
+#include "devmem.h"
 #include "errors.h"
 #include "intmath.h"
 #include "fixedsum.h"
@@ -286,6 +287,17 @@ inline uint64_t spread3(uint64_t x) {
 
 }  // namespace
 
+// Device memory of DeviceArrays.
+struct CudaMem {
+  static void *take(size_t bytes) {
+    void *p = nullptr;
+    if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+  }
+  static void give(void *p) { cudaFree(p); }
+};
+
 // Base of the per-precision contexts; the C ABI calls these.
 struct CtxBase {
   virtual ~CtxBase() {}
@@ -325,7 +337,7 @@ template <typename R>
 struct Ctx : CtxBase {
   View<R> V{};
   const Ops<R> *ops = nullptr;
-  std::vector<void *> allocs;
+  DeviceArrays<CudaMem> mem;
   double *staging = nullptr;     // (15, nc) doubles: transfers in reference order
   bool imageMesh = false;        // the grid came with periodic or symmetry images (fc2 / c2csShift / c2csXf)
   bool constrBurning = false;    // a constrained gradient (CRECONSTC 1) holds a burning injection face's row (cpOff/cpEnt)
@@ -349,38 +361,48 @@ struct Ctx : CtxBase {
     if (hostSc) cudaFreeHost(hostSc);
     if (stepGraph) cudaGraphExecDestroy(stepGraph);
     if (fixedGraph) cudaGraphExecDestroy(fixedGraph);
-    for (void *p : allocs) cudaFree(p);
     for (auto &e : chunkEv)
       if (e) cudaEventDestroy(e);
     if (copyStream) cudaStreamDestroy(copyStream);
     if (stream) cudaStreamDestroy(stream);
   }
 
-  size_t bytesHeld = 0;          // device bytes of the context's own arrays
-
   template <typename T>
   int alloc(T **p, size_t n) {
-    void *q = nullptr;
-    RFLU_CUDA(cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T)));
-    bytesHeld += std::max<size_t>(n, 1) * sizeof(T);
-    allocs.push_back(q);
+    const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+    void *q = mem.need(bytes);
+    if (!q) return noMemory(bytes);
     *p = (T *)q;
     return RFLU_OK;
   }
+  static int noMemory(size_t bytes) {
+    return fail(RFLU_ERR_CUDA, "cudaMalloc: " + std::to_string(bytes) + " bytes: " +
+                                   cudaGetErrorString(cudaErrorMemoryAllocation));
+  }
   // An array that only makes the context faster: null when the device is
-  // full, and the kernels that do without it run instead.
+  // full, and the kernels that do without it run instead.  A needed array that
+  // finds no memory takes all of them back (forgetOptional).
   template <typename T>
   bool allocOptional(T **p, size_t n) {
-    void *q = nullptr;
-    if (cudaMalloc(&q, n * sizeof(T)) != cudaSuccess) {
-      cudaGetLastError();
-      *p = nullptr;
-      return false;
-    }
-    bytesHeld += n * sizeof(T);
-    allocs.push_back(q);
-    *p = (T *)q;
-    return true;
+    *p = (T *)mem.want(n * sizeof(T));
+    return *p != nullptr;
+  }
+  template <typename T>
+  void freeOptional(T *&p) {
+    if (p) mem.release(p);
+    p = nullptr;
+  }
+  // before the optional arrays are freed: nothing that reads them is under way
+  // or captured, and no view holds them (a copy of V lives within one call,
+  // which allocates before it copies)
+  void forgetOptional() {
+    cudaStreamSynchronize(stream);
+    if (stepGraph) cudaGraphExecDestroy(stepGraph);
+    if (fixedGraph) cudaGraphExecDestroy(fixedGraph);
+    stepGraph = fixedGraph = nullptr;
+    V.fxIdx = V.fxScale = nullptr;
+    V.fxW = nullptr;
+    V.wenoW = nullptr;
   }
   template <typename T, typename S>
   int put(const T **dst, const std::vector<S> &src) {
@@ -393,9 +415,21 @@ struct Ctx : CtxBase {
     return RFLU_OK;
   }
 
-  // The fixed-point sums' arrays (View::fxIdx) on the meshes that gain from
-  // them.  The sums' scratch (seven values per cell) is the face-flux array.
-  int planFixedSums() {
+  // What only makes the context faster, after all that it needs: the WENO
+  // weights, and the fixed-point sums' arrays on the meshes that gain from them.
+  int planOptional() {
+    if (!Layout<R>::packed && V.p.reconst == 2 && V.p.spaceOrder > 1) allocOptional(&V.wenoW, 15 * (size_t)V.nc);
+    bool taken = false;
+    const int rc = planFixedSums(&taken);
+    if (!taken) {
+      freeOptional(V.fxIdx);
+      freeOptional(V.fxW);
+      freeOptional(V.fxScale);
+    }
+    return rc;
+  }
+  // The sums' scratch (seven values per cell) is the face-flux array.
+  int planFixedSums(bool *taken) {
     if (V.p.precision != RFLU_PREC_FP64 || V.p.spaceOrder < 2 || 5 * ((size_t)V.nf + V.nb) < 7 * (size_t)V.nc)
       return RFLU_OK;
     const size_t nc = V.nc;
@@ -410,12 +444,11 @@ struct Ctx : CtxBase {
     constexpr double kFixVenkatShare = 0.25;
     if (V.p.reconst == 11 && (long long)slow * 32 > kFixVenkatShare * V.nc) return RFLU_OK;
     V.fxWidth = stWidth;
-    if (!allocOptional(&V.fxW, 3 * (size_t)stWidth * nc) || !allocOptional(&V.fxIdx, (size_t)stWidth * nc)) {
-      V.fxIdx = nullptr;
+    if (!allocOptional(&V.fxW, 3 * (size_t)stWidth * nc) || !allocOptional(&V.fxIdx, (size_t)stWidth * nc))
       return RFLU_OK;
-    }
     ops->fixedSetup(V, nullptr, stream);
     RFLU_CUDA(cudaStreamSynchronize(stream));
+    *taken = true;
     return RFLU_OK;
   }
   int create(const rflu_grid_desc *g, const rflu_num_desc *num);
@@ -931,9 +964,6 @@ struct Ctx : CtxBase {
     if (!ops->vjp) return fail(RFLU_ERR_UNSUPPORTED, "rflu_gpu_unrolled_adjoint: no adjoint kernels in this precision mode");
     if (iPatch < 0 || iPatch >= nPatches) return fail(RFLU_ERR_ARG, "rflu_gpu_unrolled_adjoint: bad patch");
     if (int rc0 = ensureAdjoint()) return rc0;
-    // the whole forward and reverse sweep runs on the scratch state X
-    View<R> X;
-    if (int rc0 = scratchView(&X, false)) return rc0;
     const int nrk = V.p.nrkSteps;
     double W[6][6] = {};
     for (int t = 1; t <= nrk; ++t) W[t][t] = 1.0;
@@ -951,11 +981,17 @@ struct Ctx : CtxBase {
     // device buffers of the call: checkpoints, segment stage states, the
     // stage adjoints lambda(0..nrk), seed, VJP result, functional gradient
     const size_t nVec = (size_t)nCk + nSeg + (grad ? (size_t)nrk + 1 + 3 : 0);
-    double *buf = nullptr, *jd = nullptr;
-    RFLU_CUDA(cudaMalloc(&buf, std::max<size_t>(nVec, 1) * b5));
-    if (cudaMalloc(&jd, 3 * sizeof(double)) != cudaSuccess) {
+    double *buf = (double *)mem.takeNeeded(std::max<size_t>(nVec, 1) * b5);
+    if (!buf) return noMemory(std::max<size_t>(nVec, 1) * b5);
+    double *jd = (double *)mem.takeNeeded(3 * sizeof(double));
+    // the whole forward and reverse sweep runs on the scratch state X (taken
+    // after the allocations, which may give the optional arrays back)
+    View<R> X;
+    int rc = jd ? scratchView(&X, false) : noMemory(3 * sizeof(double));
+    if (rc) {
       cudaFree(buf);
-      return fail(RFLU_ERR_CUDA, "rflu_gpu_unrolled_adjoint: cudaMalloc");
+      cudaFree(jd);
+      return rc;
     }
     auto vec = [&](size_t k) { return buf + k * n5; };
     cudaError_t err = cudaSuccess;  // first failed copy; checked before returning
@@ -974,7 +1010,6 @@ struct Ctx : CtxBase {
     double *jStep = jd, *jAcc = jd + 1;
     cudaEvent_t ev[3];
     for (auto &e : ev) cudaEventCreate(&e);
-    int rc = RFLU_OK;
     auto finish = [&](int r) {
       for (auto &e : ev) cudaEventDestroy(e);
       cudaFree(buf);
@@ -1050,7 +1085,7 @@ struct Ctx : CtxBase {
       cudaEventElapsedTime(&b, ev[1], ev[2]);
       stats[0] = f;
       stats[1] = grad ? b : 0.0;
-      stats[2] = (double)(bytesHeld + std::max<size_t>(nVec, 1) * b5 + 3 * sizeof(double));
+      stats[2] = (double)(mem.bytes() + std::max<size_t>(nVec, 1) * b5 + 3 * sizeof(double));
       stats[3] = nCk;
     }
     return finish(syncEvents(false));
@@ -1292,6 +1327,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   const int nc = g->nCells, nf = g->nFaces, np = g->nPatches;
   const int nb = np > 0 ? g->patchFaceOff[np] : 0;
   nPatches = np;
+  mem.beforeDrop = [this] { forgetOptional(); };
   RFLU_CUDA(cudaGetDevice(&device));
   RFLU_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   RFLU_CUDA(cudaStreamCreateWithFlags(&copyStream, cudaStreamNonBlocking));
@@ -1621,7 +1657,6 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   if ((num->reconst == 1 || num->reconst == 2) && num->spaceOrder > 1 &&
       (rc = alloc(&V.gradRaw, Layout<R>::grad * (size_t)nc)))
     return rc;
-  if (!mixed && num->reconst == 2 && num->spaceOrder > 1) allocOptional(&V.wenoW, 15 * (size_t)nc);
   if ((rc = alloc(&V.rhsSum, 5 * (size_t)nc))) return rc;
   if ((rc = alloc(&V.flux, 5 * ((size_t)nf + nb)))) return rc;
   if ((rc = alloc(&V.rhs, 5 * (size_t)nc))) return rc;
@@ -1671,7 +1706,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   workBytes = sizeof(R) * (size_t)(130 * (size_t)nc + 24 * ((size_t)nf + nb) + 64) + sizeof(int) * 10 * (size_t)nc + 256;
   ops->configure(V);
   RFLU_CUDA(cudaDeviceSynchronize());
-  if ((rc = planFixedSums())) return rc;
+  if ((rc = planOptional())) return rc;
   V.tileGrid = ops->tileGrid(V, 0, &V.tileBufs);
   V.tileGridDt = ops->tileGrid(V, 1, &V.tileBufsDt);
   return checkLaunch("rflu_gpu_create");
