@@ -26,6 +26,7 @@
 #include "intmath.h"
 #include "fixedsum.h"
 #include "ops.h"
+#include "shared_slot.h"
 #include "tiles.h"
 
 namespace rflu {
@@ -355,10 +356,10 @@ struct Ctx : CtxBase {
   Scalars *sSc = nullptr;
   cudaGraphExec_t stepGraph = nullptr, fixedGraph = nullptr;
   long long lastNan = 0;
-  Scalars *hostSc = nullptr;  // pinned copy of V.sc (readScalars)
+  SharedSlot<Scalars> hostSc;  // pinned copy of V.sc (readScalars)
 
   ~Ctx() override {
-    if (hostSc) cudaFreeHost(hostSc);
+    if (hostSc.slot) cudaFreeHost(hostSc.slot);
     if (stepGraph) cudaGraphExecDestroy(stepGraph);
     if (fixedGraph) cudaGraphExecDestroy(fixedGraph);
     for (auto &e : chunkEv)
@@ -466,12 +467,14 @@ struct Ctx : CtxBase {
   }
   // The context's scalars after everything queued on the stream, through a
   // pinned copy: one wait (a pageable copy and a second wait for it cost
-  // another 10-15 us per stage of a host-driven loop).
+  // another 10-15 us per stage of a host-driven loop).  Another host thread may
+  // ask for the status meanwhile.
   int readScalars(Scalars *s) {
-    RFLU_CUDA(cudaMemcpyAsync(hostSc, V.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream));
-    RFLU_CUDA(cudaStreamSynchronize(stream));
-    *s = *hostSc;
-    return RFLU_OK;
+    return hostSc.read(s, [this](Scalars *slot) {
+      RFLU_CUDA(cudaMemcpyAsync(slot, V.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, stream));
+      RFLU_CUDA(cudaStreamSynchronize(stream));
+      return RFLU_OK;
+    });
   }
   int syncEvents(bool events) {
     if (!events) {
@@ -1661,7 +1664,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   if ((rc = alloc(&V.flux, 5 * ((size_t)nf + nb)))) return rc;
   if ((rc = alloc(&V.rhs, 5 * (size_t)nc))) return rc;
   if ((rc = alloc(&V.sc, 1))) return rc;
-  RFLU_CUDA(cudaMallocHost((void **)&hostSc, sizeof(Scalars)));
+  RFLU_CUDA(cudaMallocHost((void **)&hostSc.slot, sizeof(Scalars)));
   if ((rc = alloc(&staging, 15 * (size_t)nc + 16))) return rc;
   RFLU_CUDA(cudaMemset(V.grad, 0, sizeof(R) * Layout<R>::grad * (size_t)nc));
   RFLU_CUDA(cudaMemset(V.rhsSum, 0, sizeof(R) * 5 * (size_t)nc));
