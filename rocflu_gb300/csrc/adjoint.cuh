@@ -2077,23 +2077,6 @@ __global__ void kPatchSeed(View<R> V, AdjWork<R> W, int ip, double *Jout) {
   if (threadIdx.x == 0) *Jout = part[0];
 }
 
-// A second stream of the adjoint's launches, with the events that fork it
-// from and join it to the calling stream (created once per process).
-struct SideStream {
-  cudaStream_t stream = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
-};
-inline SideStream &sideStream() {
-  static SideStream ss = [] {
-    SideStream x;
-    cudaStreamCreateWithFlags(&x.stream, cudaStreamNonBlocking);
-    cudaEventCreateWithFlags(&x.fork, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&x.join, cudaEventDisableTiming);
-    return x;
-  }();
-  return ss;
-}
-
 template <typename R>
 struct AdjointOps {
   static void jvp(const View<R> &V, const double *cvDotRef, double *rhsDotRef, double *work, cudaStream_t s) {
@@ -2147,14 +2130,13 @@ struct AdjointOps {
   // (they write disjoint face-adjoint entries), forked from and joined
   // back to s by events, so that it fills the SMs the interior kernel's
   // last wave leaves idle.
-  static void faceAdjoint(const View<R> &V, const AdjWork<R> &W, cudaStream_t s) {
+  static void faceAdjoint(const View<R> &V, const AdjWork<R> &W, const SideStream &ss, cudaStream_t s) {
     const int nT = V.nf + V.nb;
     if (V.nf == 0 || V.nb == 0) {
       if (V.nb == 0 && nT > 0) interiorFaces(V, W, s);
       else if (nT > 0) launchOrdered(kAdjFace<R, 0>, faceShape(V, nT), s, V, W, 0, nT);
       return;
     }
-    SideStream &ss = sideStream();
     cudaEventRecord(ss.fork, s);
     cudaStreamWaitEvent(ss.stream, ss.fork, 0);
     const Shape sh = faceShape(V, V.nb);  // after an event: launched plainly
@@ -2163,7 +2145,8 @@ struct AdjointOps {
     interiorFaces(V, W, s);
     cudaStreamWaitEvent(s, ss.join, 0);
   }
-  static void vjp(const View<R> &V, const double *rhsBarRef, double *cvBarRef, double *work, cudaStream_t s) {
+  static void vjp(const View<R> &V, const double *rhsBarRef, double *cvBarRef, double *work, const SideStream &side,
+                  cudaStream_t s) {
     const size_t nT = (size_t)V.nf + V.nb;
     AdjWork<R> W = carveAdjWork<R>(work, V.nc, nT);
     // every face-adjoint entry the cell kernels read is written by the face
@@ -2171,7 +2154,7 @@ struct AdjointOps {
     if (V.p.spaceOrder > 1) gradFwd(V, W, rhsBarRef, s);
     else launchOrdered(kAdjLambda<R>, shapeFor(V, V.nc), s, V, W, rhsBarRef);
     (void)nT;
-    faceAdjoint(V, W, s);
+    faceAdjoint(V, W, side, s);
     cellAdjoint(V, W, cvBarRef, s);
   }
   static void limiterBranches(const View<R> &V, int *outRef, double *work, cudaStream_t s) {

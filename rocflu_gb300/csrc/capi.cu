@@ -346,6 +346,7 @@ struct Ctx : CtxBase {
   int tsWidthLazy = 0;           // ... and the width of its transposed-stencil weights
   int stWidth = 0;               // most stencil members of a cell
   size_t workBytes = 0;
+  SideStream side;               // made by the first adjoint call
   // scratch state (allocated by the first call that needs it): master cv,
   // dependent variables, primitive records, RK accumulator and scalars of the
   // states that the residual, tangent, adjoint, functional and diagnostic
@@ -364,6 +365,9 @@ struct Ctx : CtxBase {
     if (fixedGraph) cudaGraphExecDestroy(fixedGraph);
     for (auto &e : chunkEv)
       if (e) cudaEventDestroy(e);
+    if (side.fork) cudaEventDestroy(side.fork);
+    if (side.join) cudaEventDestroy(side.join);
+    if (side.stream) cudaStreamDestroy(side.stream);
     if (copyStream) cudaStreamDestroy(copyStream);
     if (stream) cudaStreamDestroy(stream);
   }
@@ -698,6 +702,9 @@ struct Ctx : CtxBase {
   int ensureAdjoint() {
     if (work) return RFLU_OK;
     int rc = RFLU_OK;
+    if (!side.stream) RFLU_CUDA(cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking));
+    if (!side.fork) RFLU_CUDA(cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming));
+    if (!side.join) RFLU_CUDA(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming));
     if (tsWidthLazy > 0 && !V.tsW) {
       if ((rc = alloc(&V.tsW, 4 * (size_t)tsWidthLazy * V.nc))) return rc;
       V.tsWidth = tsWidthLazy;
@@ -727,7 +734,7 @@ struct Ctx : CtxBase {
     if (rc) return rc;
     const size_t nc = V.nc;
     RFLU_CUDA(cudaMemcpyAsync(staging, rhsBar, sizeof(double) * 5 * nc, cudaMemcpyHostToDevice, stream));
-    ops->vjp(W, staging, staging + 5 * nc, work, stream);
+    ops->vjp(W, staging, staging + 5 * nc, work, side, stream);
     RFLU_CUDA(cudaMemcpyAsync(cvBar, staging + 5 * nc, sizeof(double) * 5 * nc, cudaMemcpyDeviceToHost, stream));
     return adjointDone();
   }
@@ -1067,7 +1074,7 @@ struct Ctx : CtxBase {
               }
             kStageSeed<<<nblk(V.nc), 256, 0, stream>>>(sigma, T, V.vol, V.refId, V.nc);
             loadState(seg + ((size_t)(n - n0) * nrk + st - 1) * n5);
-            ops->vjp(X, sigma, wv, work, stream);
+            ops->vjp(X, sigma, wv, work, side, stream);
             kSubInto<<<nb, 256, 0, stream>>>(lam + (size_t)(st - 1) * n5, lam + (size_t)st * n5, wv, n5);
           }
           cp(lamTop, lam, b5, cudaMemcpyDeviceToDevice);
@@ -1110,7 +1117,7 @@ struct Ctx : CtxBase {
       ops->faceFlux(V, stream);
       ops->gatherRhs(V, stream);
       cudaEventRecord(ev[1], stream);
-      ops->vjp(V, staging, staging + 5 * nc, work, stream);
+      ops->vjp(V, staging, staging + 5 * nc, work, side, stream);
       cudaEventRecord(ev[2], stream);
       RFLU_CUDA(cudaEventSynchronize(ev[2]));
       for (int k = 0; k < 2 && it > 0; ++k) {

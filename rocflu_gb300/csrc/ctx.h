@@ -89,6 +89,15 @@ template <> struct Layout<float> {
   static constexpr int prim = 8, grad = 16;
 };
 
+// A second stream of a context's adjoint launches, with the events that fork
+// it from and join it to the context's own.  One per context: contexts may run
+// in different host threads, and an event recorded again before the other
+// thread's wait was queued would order that thread's work after this one's.
+struct SideStream {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+
 template <typename R>
 struct View {
   int nc, nf, nb;             // cells, interior faces, boundary faces

@@ -26,7 +26,7 @@ struct Ops {
   int (*tileGrid)(const View<R> &, int withDt, int *bufs);  // CTAs of the persistent tiled kernels, tile buffers per CTA
   // tangent / adjoint of the residual (FP64 modes only; null elsewhere)
   void (*jvp)(const View<R> &, const double *cvDot, double *rhsDot, double *work, cudaStream_t);
-  void (*vjp)(const View<R> &, const double *rhsBar, double *cvBar, double *work, cudaStream_t);
+  void (*vjp)(const View<R> &, const double *rhsBar, double *cvBar, double *work, const SideStream &, cudaStream_t);
   void (*patchPressure)(const View<R> &, int iPatch, double *J, double *cvBar, double *work, cudaStream_t);
   // fills the adjoint's mesh-dependent arrays (View::tsW) once they exist
   void (*adjointSetup)(const View<R> &, cudaStream_t);
