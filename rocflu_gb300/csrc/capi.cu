@@ -83,10 +83,10 @@ __global__ void __launch_bounds__(kReadBlock) kReadOut(const T *src, double *dst
   const int o0 = blockIdx.x * kReadBlock, n = min(kReadBlock, nc - o0);
   if ((int)threadIdx.x < n) {
     const size_t i = newId[o0 + threadIdx.x];
-    if (kComp == 15 && kStride == 1) {  // the packed gradient record: 16 floats on a 64-byte boundary
-      T r[16];
+    if constexpr (kComp == 15 && Layout<T>::packed) {  // a gradient record: 16 floats on a 64-byte boundary
+      alignas(16) T r[16];
 #pragma unroll
-      for (int k = 0; k < 16; k += 16 / (int)sizeof(T))
+      for (int k = 0; k < 16; k += 4)
         *reinterpret_cast<int4 *>(r + k) = *reinterpret_cast<const int4 *>(src + 16 * i + k);
 #pragma unroll
       for (int k = 0; k < kComp; ++k) s[threadIdx.x * kComp + k] = (double)r[k];
