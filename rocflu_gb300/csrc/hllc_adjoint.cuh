@@ -107,7 +107,7 @@ __host__ __device__ inline void hllc2Adjoint(T g, T nx, T ny, T nz, T nm, const 
   if (slRoe) { qsb += slb; asb -= slb; } else { qlb += slb; alb = -slb; }
   if (srRoe) { qsb += srb; asb += srb; } else { qrb += srb; arb = srb; }
   // Roe averages: as = sqrt(g1 (Hs - |us|^2/2)), Xs = w2 (Xl + w1 Xr)
-  const T Hsb = nonZero_(asb) ? div_(half * g1 * asb, as) : T(0);
+  const T Hsb = nonZero_(asb) && pos_(as) ? div_(half * g1 * asb, as) : T(0);
   const T usb = -Hsb * us, vsb = -Hsb * vs, wsb = -Hsb * ws;
   const T w1b = w2 * (usb * (ur - us) + vsb * (vr - vs) + wsb * (wr - ws) + qsb * (qr - qs) + Hsb * (Hr - Hs));
   const T w12 = w2 * w1;
@@ -123,8 +123,9 @@ __host__ __device__ inline void hllc2Adjoint(T g, T nx, T ny, T nz, T nm, const 
   plb += Hlb * irl;
   prb += Hrb * irr;
   const T ha = half * alb * al, hb = half * arb * ar;
-  plb += div_(ha, pl);
-  prb += div_(hb, pr);
+  // a root at zero (p = 0) counts as a derivative of zero, as in dual.cuh
+  if (nonZero_(ha)) plb += div_(ha, pl);
+  if (nonZero_(hb)) prb += div_(hb, pr);
   const T ig1 = div_(T(1), g1);
   plb += elb * irL * ig1;
   prb += erb * irR * ig1;
