@@ -1976,7 +1976,7 @@ __global__ void __launch_bounds__(kBlock) kAdjCell2(View<R> V, AdjWork<R> W, dou
     const double b1 = W.dvbar[n + j], b2 = W.dvbar[2 * n + j];
     if (nonZero_(b1) || nonZero_(b2)) {
       const double t = div_((g - 1.0) * (ir * V.cv[4 * n + j] - ke), gc), c = sqrt_(g * gc * t);
-      const double tb = b1 + div_(0.5 * g * gc * b2, c);
+      const double tb = pos_(c) ? b1 + div_(0.5 * g * gc * b2, c) : b1;  // a root at zero: derivative 0 (dual.cuh)
       pb += div_(tb * ir, gc);
       rb = -(tb * t * ir);  // dT/drho at fixed p
     }
