@@ -615,16 +615,25 @@ struct Ctx : CtxBase {
     if (rc) return rc;
     return syncEvents(true);
   }
+  // The view whose launches are captured.
+  View<R> graphView() const {
+    View<R> G = V;
+    G.overlap = V.nc <= overlapLimit(Layout<R>::packed, true);
+    return G;
+  }
   // One time step (dt + all stages + time advance) captured once as a graph.
   int ensureStepGraph() {
     if (stepGraph) return RFLU_OK;
     cudaGraph_t graph;
+    const View<R> G = graphView();
     RFLU_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    ops->stepStart(V, stream);  // dt reduction + gradients of stage 1
-    ops->faceFlux(V, stream);
-    ops->gatherUpdate(V, 1, &V.sc->dtMin, stream);
-    for (int s = 2; s <= V.p.nrkSteps; ++s) stageKernels(s);
-    ops->stepEnd(V, stream);
+    ops->stepStart(G, stream);  // dt reduction + gradients of stage 1
+    View<R> F = G;  // after kDtFinalize's one thread, but for the FP64 modes' gradients
+    if (Layout<R>::packed || V.p.spaceOrder < 2) F.overlap = 1;
+    ops->faceFlux(F, stream);
+    ops->gatherUpdate(G, 1, &G.sc->dtMin, stream);
+    for (int s = 2; s <= V.p.nrkSteps; ++s) stageKernelsOf(G, s);
+    ops->stepEnd(G, stream);
     RFLU_CUDA(cudaStreamEndCapture(stream, &graph));
     cudaError_t e = cudaGraphInstantiate(&stepGraph, graph, 0);
     cudaGraphDestroy(graph);
@@ -634,8 +643,9 @@ struct Ctx : CtxBase {
   int ensureFixedGraph() {
     if (fixedGraph) return RFLU_OK;
     cudaGraph_t graph;
+    const View<R> G = graphView();
     RFLU_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    for (int s = 1; s <= V.p.nrkSteps; ++s) stageKernels(s);
+    for (int s = 1; s <= V.p.nrkSteps; ++s) stageKernelsOf(G, s);
     RFLU_CUDA(cudaStreamEndCapture(stream, &graph));
     cudaError_t e = cudaGraphInstantiate(&fixedGraph, graph, 0);
     cudaGraphDestroy(graph);
@@ -1527,6 +1537,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
 
   // ---- device upload -----------------------------------------------------------
   V.nc = nc; V.nf = nf; V.nb = nb;
+  V.overlap = nc <= overlapLimit(mixed, false);
   RFLU_CUDA(cudaDeviceGetAttribute(&V.sms, cudaDevAttrMultiProcessorCount, device));
   int rc = 0;
 #define PUT(dst, src, T) if ((rc = put<T>(&(dst), src))) return rc

@@ -98,10 +98,18 @@ struct SideStream {
   cudaEvent_t fork = nullptr, join = nullptr;
 };
 
+// The cells up to which every launch overlaps the kernel before, launched from
+// the host and captured in a graph (kernels.cuh: launchOrdered, where both sides
+// of each line stand).
+constexpr int overlapLimit(bool mixed, bool captured) {
+  return captured ? (mixed ? 6000 : 2000) : (mixed ? 33000 : 10000);
+}
+
 template <typename R>
 struct View {
   int nc, nf, nb;             // cells, interior faces, boundary faces
   int sms;                    // SMs of the device (launch shapes)
+  int overlap;                // launches overlap the kernel before (launchOrdered)
   // interior faces (storage order), renumbered cells; FP64 modes
   const int *fc1, *fc2;
   const R *fnx, *fny, *fnz, *fnm;   // unit normal and area

@@ -61,16 +61,39 @@ inline Shape shapeFor(const View<R> &V, long long n) {
 // through the non-coherent path (ld.global.nc), whose data have to be constant
 // over the kernel's whole lifetime.  Kernels that follow another stream's event
 // are launched plainly.
-// Measured: 4 unrolled mixed steps of 32,768
-// cells with their gradient 2.56 -> 2.32 ms, 40 FP64 steps of 6,400 cells 3.04 ->
-// 3.01; on meshes of many waves the waiting blocks cost more than they hide (10
-// mixed steps of 2.1 M cells 15.9 -> 18.6 ms), so grids above kOverlapThreads
-// are launched plainly.
+//
+// Which launches overlap (View::overlap, overlapLimit): waiting blocks are
+// placed beside the running ones, wherever these leave room, and an uneven
+// placement lasts for the whole kernel.  Launched from the host, a small mesh's
+// kernels are bound by the launches and gain; replayed in a graph they have
+// little launch to hide, and meshes of some blocks per SM lose.  A kernel of one
+// thread, or after one, always overlaps: nothing is in its blocks' way.
+// Without -> with overlap on every launch, a graph's step: mixed WENO 4,096
+// cells 84.7 -> 78.6 us, 8,000 cells 88.8 -> 89.7, 32,768 cells 86.8 -> 116;
+// mixed Barth-Jespersen 4,096 cells 66.4 -> 64.5, 8,000 cells 71.0 -> 80.3; FP64
+// Barth-Jespersen 1,728 cells 239.6 -> 237.5, 4,096 cells 215 -> 223, 32,768
+// cells 297 -> 407.  With only the launches beside one thread: the 6,400-cell
+// shock tube 70.1 -> 68.2, the 25,600-cell one 107.3 -> 105.2 (106.4 with all).
+// Launched from the host: three stages of 4,096 mixed cells 92 -> 69 us, of
+// 32,768 90 -> 80, of 125,000 153 -> 165; FP64 4,096 cells 216 -> 190, WENO of
+// 13,824 cells 284 -> 315; VJPs of tetrahedra (WENO), 34,992 mixed 220 -> 236,
+// 34,992 FP64 817 -> 988; two unrolled mixed steps of 32,768 cells with their
+// gradient 1318 -> 1201.
 __device__ inline void gridOrder() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-constexpr size_t kOverlapThreads = 1 << 17;
+template <typename R, typename... A>
+inline bool overlaps(const View<R> &V, const A &...) {
+  return V.overlap != 0;
+}
+// The view for a launch right after a kernel of one thread.
+template <typename R>
+inline View<R> afterOne(const View<R> &V) {
+  View<R> W = V;
+  W.overlap = 1;
+  return W;
+}
 template <typename... P, typename... A>
 inline void launchOrdered(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg{};
@@ -82,7 +105,8 @@ inline void launchOrdered(void (*kernel)(P...), dim3 grid, dim3 block, size_t sm
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = (size_t)grid.x * grid.y * block.x <= kOverlapThreads ? 1 : 0;
+  const bool one = (size_t)grid.x * grid.y * block.x == 1;
+  cfg.numAttrs = one || overlaps(args...) ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 template <typename... P, typename... A>
@@ -1441,8 +1465,9 @@ inline FixFields fixFields(double *scratch, size_t nc) {
 __device__ inline unsigned fixExpOf(unsigned long long w, int v) { return (unsigned)(w >> (10 * v)) & 1023u; }
 
 template <typename R>
-__global__ void __launch_bounds__(kBlock) kFixRecords(const R *q, FixFields F, int nc) {
+__global__ void __launch_bounds__(kBlock) kFixRecords(View<R> V, const R *q, FixFields F) {
   gridOrder();
+  const int nc = V.nc;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nc) return;
   unsigned long long w = 0;
@@ -3260,7 +3285,7 @@ struct Launch {
   static void launchFixed(const View<R> &V, const R *q, R *out, bool primal, cudaStream_t s) {
     if constexpr (kFixedSums && !Layout<R>::packed) {
       const FixFields F = fixFields(V.flux, V.nc);
-      launchOrdered(kFixRecords<R>, shapeFor(V, V.nc), s, q, F, V.nc);
+      launchOrdered(kFixRecords<R>, shapeFor(V, V.nc), s, V, q, F);
       launchOrdered(kFixExponents<R>, shapeFor(V, V.nc), s, V, F);
       const int b = std::min(kFixBlock, shapeFor(V, V.nc).block);
       launchOrdered(kGradFixed<R>, dim3((V.nc + b - 1) / b), dim3(b), 0, s, V, q, F, out, primal);
@@ -3401,10 +3426,11 @@ struct Launch {
   // mode: the FP32 sum from the primitive state, as its steps take it.
   static void timestep(const View<R> &V, cudaStream_t s) {
     launchOrdered(kStepBegin<R>, dim3(1), dim3(1), 0, s, V);
-    if (Ref<R>::on) launchOrdered(kCellDt<R>, shapeFor(V, V.nc), s, V);
+    const View<R> W = afterOne(V);
+    if (Ref<R>::on) launchOrdered(kCellDt<R>, shapeFor(V, V.nc), s, W);
     else if (Layout<R>::packed && V.tiled)
-      launchOrdered(kCellDtTile<R>, dim3((V.nc + kTile - 1) / kTile), dim3(kBlock), dtTileSmemBytes(V), s, V);
-    else launchOrdered(kCellDtPrim<R>, shapeFor(V, V.nc), s, V);
+      launchOrdered(kCellDtTile<R>, dim3((V.nc + kTile - 1) / kTile), dim3(kBlock), dtTileSmemBytes(V), s, W);
+    else launchOrdered(kCellDtPrim<R>, shapeFor(V, V.nc), s, W);
     launchOrdered(kDtFinalize<R>, dim3(1), dim3(1), 0, s, V);
   }
   // Time-step reduction + gradients of the first stage of a step.  The FP64
@@ -3417,7 +3443,7 @@ struct Launch {
       gradLimit(V, s);
     } else {
       launchOrdered(kStepBegin<R>, dim3(1), dim3(1), 0, s, V);
-      const View<R> W = rawView(V);
+      const View<R> W = afterOne(rawView(V));
       if (V.tiled) launchTile<true>(W, s);
       else launchOrdered(kGradLimitDt<R>, shapeFor(V, V.nc), s, W);
       if (weno(V) && V.p.spaceOrder > 1) smooth(V, s);
