@@ -2091,7 +2091,7 @@ struct AdjointOps {
     } else if (V.p.spaceOrder > 1) {
       const bool haveG = Launch<R>::fixedSums(V);
       if (haveG) {
-        Launch<R>::launchFixed(V, V.prim, W.G, true, s);
+        unlimited(V, W, s);
         Launch<R>::launchFixed(V, W.primd, W.Gbar, false, s);
       }
       launchOrdered(kTanGrad<R>, shapeFor(V, V.nc), s, V, W, haveG);
@@ -2100,9 +2100,16 @@ struct AdjointOps {
     launchOrdered(kTanFlux<R>, faceShape(V, nT), s, V, W);
     launchOrdered(kTanGather<R>, shapeFor(V, V.nc), s, V, W, rhsDotRef);
   }
+  // The unlimited gradients into W.G.  The derivatives of the WENO averages form
+  // all weights themselves, so the view's are not stored (15 divisions a cell).
+  static void unlimited(const View<R> &V, const AdjWork<R> &W, cudaStream_t s) {
+    View<R> X = V;
+    X.wenoW = nullptr;
+    Launch<R>::launchFixed(X, V.prim, W.G, true, s);
+  }
   static void gradFwd(const View<R> &V, const AdjWork<R> &W, const double *lamRef, cudaStream_t s) {
     const bool haveG = Launch<R>::fixedSums(V);
-    if (haveG) Launch<R>::launchFixed(V, V.prim, W.G, true, s);
+    if (haveG) unlimited(V, W, s);
     if (V.p.reconst == 10) launchOrdered(kAdjGradFwd<R, true>, shapeFor(V, V.nc), s, V, W, lamRef, haveG);
     else launchOrdered(kAdjGradFwd<R, false>, shapeFor(V, V.nc), s, V, W, lamRef, haveG);
     if (isWeno(V.p)) {
