@@ -1799,9 +1799,8 @@ __global__ void __launch_bounds__(kBlock) kAdjCell2(View<R> V, AdjWork<R> W, dou
     } else {
       // In the FP64 mode (kFixedSums) four entries' products are summed by
       // FMAs before they reach the cell's sum: 65 FP64 instructions instead of
-      // 80, and fewer roundings at the sum's size (error against 128 bits over
-      // 16 to 60 entries 0.5 to 0.95 of the entry-by-entry sum's).  196,608
-      // tetrahedra: 548 -> 514 us.
+      // 80, and fewer roundings at the sum's size.  196,608 tetrahedra: 548 ->
+      // 514 us.
       const int end = V.tsOff[j + 1];
       constexpr int kGroup = kFixedSums ? 4 : 1;
       for (int e0 = V.tsOff[j]; e0 < end; e0 += kGroup) {

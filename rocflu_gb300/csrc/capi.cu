@@ -346,7 +346,7 @@ struct Ctx : CtxBase {
   int tsWidthLazy = 0;           // ... and the width of its transposed-stencil weights
   int stWidth = 0;               // most stencil members of a cell
   size_t workBytes = 0;
-  SideStream side;               // made by the first adjoint call
+  SideStream side;               // the copy stream, which no transfer uses meanwhile
   // scratch state (allocated by the first call that needs it): master cv,
   // dependent variables, primitive records, RK accumulator and scalars of the
   // states that the residual, tangent, adjoint, functional and diagnostic
@@ -367,7 +367,6 @@ struct Ctx : CtxBase {
       if (e) cudaEventDestroy(e);
     if (side.fork) cudaEventDestroy(side.fork);
     if (side.join) cudaEventDestroy(side.join);
-    if (side.stream) cudaStreamDestroy(side.stream);
     if (copyStream) cudaStreamDestroy(copyStream);
     if (stream) cudaStreamDestroy(stream);
   }
@@ -618,7 +617,7 @@ struct Ctx : CtxBase {
   // The view whose launches are captured.
   View<R> graphView() const {
     View<R> G = V;
-    G.overlap = V.nc <= overlapLimit(Layout<R>::packed, true);
+    G.overlap = V.nc <= overlapLimit(Layout<R>::packed, V.p.spaceOrder, true);
     return G;
   }
   // One time step (dt + all stages + time advance) captured once as a graph.
@@ -712,9 +711,6 @@ struct Ctx : CtxBase {
   int ensureAdjoint() {
     if (work) return RFLU_OK;
     int rc = RFLU_OK;
-    if (!side.stream) RFLU_CUDA(cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking));
-    if (!side.fork) RFLU_CUDA(cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming));
-    if (!side.join) RFLU_CUDA(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming));
     if (tsWidthLazy > 0 && !V.tsW) {
       if ((rc = alloc(&V.tsW, 4 * (size_t)tsWidthLazy * V.nc))) return rc;
       V.tsWidth = tsWidthLazy;
@@ -1352,6 +1348,9 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
   RFLU_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   RFLU_CUDA(cudaStreamCreateWithFlags(&copyStream, cudaStreamNonBlocking));
   for (auto &e : chunkEv) RFLU_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  side.stream = copyStream;
+  RFLU_CUDA(cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming));
+  RFLU_CUDA(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming));
 
   // ---- renumbering: Morton order of the cell centroids --------------------
   double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
@@ -1537,7 +1536,7 @@ int Ctx<R>::create(const rflu_grid_desc *g, const rflu_num_desc *num) {
 
   // ---- device upload -----------------------------------------------------------
   V.nc = nc; V.nf = nf; V.nb = nb;
-  V.overlap = nc <= overlapLimit(mixed, false);
+  V.overlap = nc <= overlapLimit(mixed, num->spaceOrder, false);
   RFLU_CUDA(cudaDeviceGetAttribute(&V.sms, cudaDevAttrMultiProcessorCount, device));
   int rc = 0;
 #define PUT(dst, src, T) if ((rc = put<T>(&(dst), src))) return rc

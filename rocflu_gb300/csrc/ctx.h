@@ -101,8 +101,9 @@ struct SideStream {
 // The cells up to which every launch overlaps the kernel before, launched from
 // the host and captured in a graph (kernels.cuh: launchOrdered, where both sides
 // of each line stand).
-constexpr int overlapLimit(bool mixed, bool captured) {
-  return captured ? (mixed ? 6000 : 2000) : (mixed ? 33000 : 10000);
+constexpr int overlapLimit(bool mixed, int spaceOrder, bool captured) {
+  if (mixed) return captured ? 6000 : 33000;
+  return !captured ? 10000 : spaceOrder < 2 ? 16000 : 2000;
 }
 
 template <typename R>

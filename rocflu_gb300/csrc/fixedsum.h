@@ -156,10 +156,12 @@ RFLU_HD inline int64_t fixWeight(double w, int eMax) {
 // jittered tetrahedra (40), smooth, random and discontinuous fields, in units of
 // sum |w||d|: root mean square of cubic cells 2e-17 to 7e-17 (hexahedra) and
 // 2e-17 to 1.1e-16 (tetrahedra) against the FP64 sum's 5e-17 to 1.1e-16 and
-// 6e-17 to 1.4e-16 (largest 2.9e-16 and 8.9e-16 against 6.2e-16 and 8.5e-16); of cells of aspect 2 at most the FP64 sum's.  Beyond, the
-// fixed point falls behind: aspect 8 in x 5e-16 against 1.2e-16, aspect 1e4
-// 5e-13.
-constexpr int kFixCompSpread = 2, kFixMemberSpread = 5;
+// 6e-17 to 1.4e-16 (largest 2.9e-16 and 8.9e-16 against 6.2e-16 and 8.5e-16); of
+// cells of aspect 2 at most the FP64 sum's.  Beyond, the fixed point falls
+// behind: aspect 8 in x 5e-16 against 1.2e-16, aspect 1e4 5e-13.  (Members up to
+// 2^5 apart would leave out 11 of 196,608 jittered tetrahedra, whose warps'
+// FP64 loops held up every launch: tangent and adjoint 2595 -> 2681 us.)
+constexpr int kFixCompSpread = 2, kFixMemberSpread = 6;
 constexpr int kFixNoWeights = -1;
 template <typename R>
 RFLU_HD inline int fixCellWeights(const R *wx, const R *wy, const R *wz, int n) {

@@ -72,8 +72,9 @@ inline Shape shapeFor(const View<R> &V, long long n) {
 // cells 84.7 -> 78.6 us, 8,000 cells 88.8 -> 89.7, 32,768 cells 86.8 -> 116;
 // mixed Barth-Jespersen 4,096 cells 66.4 -> 64.5, 8,000 cells 71.0 -> 80.3; FP64
 // Barth-Jespersen 1,728 cells 239.6 -> 237.5, 4,096 cells 215 -> 223, 32,768
-// cells 297 -> 407.  With only the launches beside one thread: the 6,400-cell
-// shock tube 70.1 -> 68.2, the 25,600-cell one 107.3 -> 105.2 (106.4 with all).
+// cells 297 -> 407; first order 6,400 cells 70.1 -> 68.2, 12,800 cells (40 steps)
+// 3375 -> 3290, with only the launches beside one thread 3330; 25,600 cells 4443
+// -> 4393, with only those 4361.
 // Launched from the host: three stages of 4,096 mixed cells 92 -> 69 us, of
 // 32,768 90 -> 80, of 125,000 153 -> 165; FP64 4,096 cells 216 -> 190, WENO of
 // 13,824 cells 284 -> 315; VJPs of tetrahedra (WENO), 34,992 mixed 220 -> 236,

@@ -39,13 +39,13 @@ def stencil_weights(s):
 
 def in_fixed_point(s, w):
     """The cells whose weights are of like size: the exponents of the components' largest within 2 of each other,
-    those of the members' largest within 5."""
+    those of the members' largest within 6."""
     e = np.frexp(np.abs(w))[1]
     e = np.where(w == 0, -2000, e)
     off = s.c2cs_off[:-1]
     comp, member = np.maximum.reduceat(e, off), e.max(axis=1)
     return (member.max() < 600) & (np.ptp(comp, axis=1) <= 2) & \
-        (np.maximum.reduceat(member, off) - np.minimum.reduceat(member, off) <= 5)
+        (np.maximum.reduceat(member, off) - np.minimum.reduceat(member, off) <= 6)
 
 
 def stretched(mesh, aspect):
