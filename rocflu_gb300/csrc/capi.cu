@@ -404,7 +404,7 @@ struct Ctx : CtxBase {
     if (stepGraph) cudaGraphExecDestroy(stepGraph);
     if (fixedGraph) cudaGraphExecDestroy(fixedGraph);
     stepGraph = fixedGraph = nullptr;
-    V.fxIdx = V.fxScale = nullptr;
+    V.fxIdx = V.fxTop = nullptr;
     V.fxW = nullptr;
     V.wenoW = nullptr;
   }
@@ -428,7 +428,7 @@ struct Ctx : CtxBase {
     if (!taken) {
       freeOptional(V.fxIdx);
       freeOptional(V.fxW);
-      freeOptional(V.fxScale);
+      freeOptional(V.fxTop);
     }
     return rc;
   }
@@ -437,7 +437,7 @@ struct Ctx : CtxBase {
     if (V.p.precision != RFLU_PREC_FP64 || V.p.spaceOrder < 2 || 5 * ((size_t)V.nf + V.nb) < 7 * (size_t)V.nc)
       return RFLU_OK;
     const size_t nc = V.nc;
-    if (stWidth < 1 || stWidth > kFixMaxTerms || !allocOptional(&V.fxScale, nc)) return RFLU_OK;
+    if (stWidth < 1 || stWidth > kFixMaxTerms || !allocOptional(&V.fxTop, nc)) return RFLU_OK;
     int slow = 0, *dev = reinterpret_cast<int *>(staging);
     RFLU_CUDA(cudaMemsetAsync(dev, 0, sizeof(int), stream));
     ops->fixedSetup(V, dev, stream);

@@ -102,8 +102,8 @@ struct SideStream {
 // the host and captured in a graph (kernels.cuh: launchOrdered, where both sides
 // of each line stand).
 constexpr int overlapLimit(bool mixed, int spaceOrder, bool captured) {
-  if (mixed) return captured ? 6000 : 33000;
-  return !captured ? 10000 : spaceOrder < 2 ? 16000 : 2000;
+  if (mixed) return captured ? 4500 : 33000;
+  return !captured ? 10000 : spaceOrder < 2 ? 16000 : 3600;
 }
 
 template <typename R>
@@ -156,11 +156,11 @@ struct View {
   // RFLU_PREC_FP64: the stencil entry-major (entry k of cell i at k*nc + i)
   // for the fixed-point sums (fixedsum.h): member (-1 past the end), the
   // weights' halves (component c at (c*fxWidth + k)*nc + i) in units of
-  // 2^(e - 1077) with e the component's exponent in the cell's packed
-  // fxScale (fixCellWeights); null: the FP64 sums
+  // 2^(fxTop - 1077), fxTop the exponent of the cell's largest weight
+  // (fixCellWeights); null: the FP64 sums
   int *fxIdx;
   int2 *fxW;
-  int *fxScale;
+  int *fxTop;
   int fxWidth;
   R *wSum;                          // FP64 layouts: each cell's sum of them (3, nc), for the adjoint
   const double *vol;

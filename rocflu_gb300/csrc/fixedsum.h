@@ -143,24 +143,24 @@ RFLU_HD inline int64_t fixWeight(double w, int eMax) {
   return s == 0 ? f.m : ((f.m >> (s - 1)) + 1) >> 1;
 }
 
-// The three components of a cell's least-squares weights are blocks of their
-// own: their largest exponents, ten bits each (kFixEmin taken as 1), or
-// kFixNoWeights where the cell's sums stay in FP64.
+// The exponent of the largest of a cell's least-squares weights, their block's,
+// or kFixNoWeights where the cell's sums stay in FP64.
 //
-// A weight is rounded to 2^-56 of its component's largest, so a cell loses
-// digits where its weights differ widely: a member whose weights are all small
-// carries a large difference on a stretched cell, and FP64 keeps its product's
-// digits.  The sums take the cells whose components' largest weights lie within
-// kFixCompSpread exponents of each other and whose members' largest weights
-// within kFixMemberSpread.  Error against 128 bits on hexahedra (26 members) and
-// jittered tetrahedra (40), smooth, random and discontinuous fields, in units of
-// sum |w||d|: root mean square of cubic cells 2e-17 to 7e-17 (hexahedra) and
-// 2e-17 to 1.1e-16 (tetrahedra) against the FP64 sum's 5e-17 to 1.1e-16 and
-// 6e-17 to 1.4e-16 (largest 2.9e-16 and 8.9e-16 against 6.2e-16 and 8.5e-16); of
-// cells of aspect 2 at most the FP64 sum's.  Beyond, the fixed point falls
-// behind: aspect 8 in x 5e-16 against 1.2e-16, aspect 1e4 5e-13.  (Members up to
-// 2^5 apart would leave out 11 of 196,608 jittered tetrahedra, whose warps'
-// FP64 loops held up every launch: tangent and adjoint 2595 -> 2681 us.)
+// A weight is rounded to 2^-56 of the block's largest, so a cell loses digits
+// where its weights differ widely: those along a cell's long axis are smaller by
+// its aspect ratio, and a member whose weights are all small carries a large
+// difference, whose product's digits FP64 keeps.  The sums take the cells whose
+// components' largest weights lie within kFixCompSpread exponents of each other
+// and whose members' largest weights within kFixMemberSpread.  Error against 128
+// bits on hexahedra (26 members) and jittered tetrahedra (40), smooth, random and
+// discontinuous fields, in units of sum |w||d|: root mean square of cubic cells
+// 2e-17 to 7e-17 (hexahedra) and 2e-17 to 1.1e-16 (tetrahedra) against the FP64
+// sum's 5e-17 to 1.1e-16 and 6e-17 to 1.4e-16 (largest 2.9e-16 and 8.9e-16 against
+// 6.2e-16 and 8.5e-16); of cells of aspect 2 at most the FP64 sum's.  Beyond, the
+// fixed point falls behind: aspect 8 in x 5e-16 against 1.2e-16, aspect 1e4
+// 5e-13, with an exponent per component too.  (Members up to 2^5 apart would
+// leave out 11 of 196,608 jittered tetrahedra, whose warps' FP64 loops held up
+// every launch: tangent and adjoint 2595 -> 2681 us.)
 constexpr int kFixCompSpread = 2, kFixMemberSpread = 6;
 constexpr int kFixNoWeights = -1;
 template <typename R>
@@ -177,12 +177,10 @@ RFLU_HD inline int fixCellWeights(const R *wx, const R *wy, const R *wz, int n) 
   }
   int least = e[0] < e[1] ? e[0] : e[1];
   least = e[2] < least ? e[2] : least;
-  if (n < 1 || n > kFixMaxTerms || fixScale(top) == kFixBadScale || fixScale(least) == kFixBadScale ||
-      top - least > kFixCompSpread || top - low > kFixMemberSpread)
+  if (n < 1 || n > kFixMaxTerms || fixScale(top) == kFixBadScale || top - least > kFixCompSpread ||
+      top - low > kFixMemberSpread)
     return kFixNoWeights;
-  return (e[0] - kFixEmin + 1) | (e[1] - kFixEmin + 1) << 10 | (e[2] - kFixEmin + 1) << 20;
+  return top;
 }
-// Component c's largest exponent, and its scale.
-RFLU_HD inline int fixWeightExp(int packed, int c) { return (packed >> (10 * c) & 1023) + kFixEmin - 1; }
 
 }  // namespace rflu

@@ -68,13 +68,13 @@ inline Shape shapeFor(const View<R> &V, long long n) {
 // kernels are bound by the launches and gain; replayed in a graph they have
 // little launch to hide, and meshes of some blocks per SM lose.  A kernel of one
 // thread, or after one, always overlaps: nothing is in its blocks' way.
-// Without -> with overlap on every launch, a graph's step: mixed WENO 4,096
-// cells 84.7 -> 78.6 us, 8,000 cells 88.8 -> 89.7, 32,768 cells 86.8 -> 116;
-// mixed Barth-Jespersen 4,096 cells 66.4 -> 64.5, 8,000 cells 71.0 -> 80.3; FP64
-// Barth-Jespersen 1,728 cells 239.6 -> 237.5, 4,096 cells 215 -> 223, 32,768
-// cells 297 -> 407; first order 6,400 cells 70.1 -> 68.2, 12,800 cells (40 steps)
-// 3375 -> 3290, with only the launches beside one thread 3330; 25,600 cells 4443
-// -> 4393, with only those 4361.
+// Without -> with overlap on every launch, in graphs: six mixed WENO steps of
+// 4,096 cells 617 -> 594 us, of 4,913 cells 638 -> 645, of 32,768 cells 707 ->
+// 895; six mixed Barth-Jespersen steps of 2,744 cells 530 -> 516, of 4,913 cells
+// 534 -> 566, of 8,000 cells 568 -> 658; six FP64 ones of 3,375 cells 1524 ->
+// 1442, of 4,096 cells 1363 -> 1409, of 32,768 cells 1952 -> 2619; 40 first-order
+// FP64 steps of 6,400 cells 2808 -> 2728, of 12,800 cells 3375 -> 3290 (with only
+// the launches beside one thread 3330), of 25,600 cells 4443 -> 4393 (4361).
 // Launched from the host: three stages of 4,096 mixed cells 92 -> 69 us, of
 // 32,768 90 -> 80, of 125,000 153 -> 165; FP64 4,096 cells 216 -> 190, WENO of
 // 13,824 cells 284 -> 315; VJPs of tetrahedra (WENO), 34,992 mixed 220 -> 236,
@@ -1425,8 +1425,7 @@ __device__ inline void cpAsync8(void *smemDst, const void *gSrc) {
 // Measured, 421,875 hexahedra of 26 members, FP64 pipe 100% busy before: about
 // 440 us of the gradient kernel -> 235 us in the three kernels below; 131,712
 // tetrahedra of 40: 260 -> 132 us.  The block whose largest magnitude sets the
-// unit is, for the values, the cell's own stencil and variable, for the weights
-// its component.  The rounding, 2^-55 of the largest value the fit sees and
+// unit is the cell's own stencil, for the values per variable.  The rounding, 2^-55 of the largest value the fit sees and
 // 2^-56 of the largest weight, is below that of the FP64 differences and partial
 // sums while the weights are of like size (fixCellWeights: cells up to about
 // twice as long as wide); the gradient of a cell is meant as a vector, a
@@ -1505,7 +1504,7 @@ __global__ void __launch_bounds__(kBlock) kFixExponents(View<R> V, FixFields F) 
   F.eMax[i] = w;
 }
 
-// The exponents of each cell's weights (View::fxScale, fixCellWeights) and the
+// The exponent of each cell's weights (View::fxTop, fixCellWeights) and the
 // number of warps that hold a cell whose sums stay in FP64: its own weights say
 // so, or a member seen reflected.
 template <typename R>
@@ -1515,12 +1514,12 @@ __global__ void __launch_bounds__(kBlock) kFixCells(View<R> V, int *slow) {
   bool fp64 = false;
   if (i < V.nc) {
     const int sb = V.stOff[i], n = V.stOff[i + 1] - sb;
-    int packed = fixCellWeights(V.wx + sb, V.wy + sb, V.wz + sb, n);
+    int top = fixCellWeights(V.wx + sb, V.wy + sb, V.wz + sb, n);
     if (V.stXf)
       for (int s = sb; s < sb + n; ++s)
-        if (V.stXf[s] >= 0) packed = kFixNoWeights;
-    V.fxScale[i] = packed;
-    fp64 = packed == kFixNoWeights;
+        if (V.stXf[s] >= 0) top = kFixNoWeights;
+    V.fxTop[i] = top;
+    fp64 = top == kFixNoWeights;
   }
   if (__any_sync(0xffffffffu, fp64) && (threadIdx.x & 31) == 0) atomicAdd(slow, 1);
 }
@@ -1533,15 +1532,15 @@ __global__ void __launch_bounds__(kBlock) kFixWeights(View<R> V) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.nc) return;
   const size_t n = V.nc;
-  const int sb = V.stOff[i], cnt = V.stOff[i + 1] - sb, packed = V.fxScale[i];
+  const int sb = V.stOff[i], cnt = V.stOff[i + 1] - sb, top = V.fxTop[i];
   for (int k = 0; k < V.fxWidth; ++k) {
     const bool on = k < cnt;
     V.fxIdx[k * n + i] = on ? V.stIdx[sb + k] : -1;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       FixHalves h{0, 0};
-      if (on && packed != kFixNoWeights)
-        h = fixSplit(fixWeight((double)(c == 0 ? V.wx : c == 1 ? V.wy : V.wz)[sb + k], fixWeightExp(packed, c)));
+      if (on && top != kFixNoWeights)
+        h = fixSplit(fixWeight((double)(c == 0 ? V.wx : c == 1 ? V.wy : V.wz)[sb + k], top));
       V.fxW[(c * (size_t)V.fxWidth + k) * n + i] = make_int2(h.hi, h.lo);
     }
   }
@@ -1563,9 +1562,9 @@ __global__ void __launch_bounds__(kFixBlock, 3) kGradFixed(View<R> V, const R *q
   unsigned emax[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) emax[v] = fixExpOf(ew, v);
-  const int packed = V.fxScale[i];
+  const int top = V.fxTop[i];
   R g[15];
-  if (packed != kFixNoWeights && max(max(max(emax[0], emax[1]), max(emax[2], emax[3])), emax[4]) != kFixExpBad) {
+  if (top != kFixNoWeights && max(max(max(emax[0], emax[1]), max(emax[2], emax[3])), emax[4]) != kFixExpBad) {
     // a cell's five values in units of the stencil's exponents: the ten-bit
     // differences of all five come from one subtraction (no field borrows)
     auto load = [&](int j, long long *m, unsigned long long &e) {
@@ -1636,8 +1635,7 @@ __global__ void __launch_bounds__(kFixBlock, 3) kGradFixed(View<R> V, const R *q
       fetch(k + kFixDepth);  // into the slot just read
     }
 #pragma unroll
-    for (int k = 0; k < 15; ++k)
-      g[k] = (R)fixResult(a[k], fixScale(fixWeightExp(packed, k % 3)) - 55 + (int)emax[k / 3] + kFixEmin - 1 - 1077);
+    for (int k = 0; k < 15; ++k) g[k] = (R)fixResult(a[k], fixScale(top) - 55 + (int)emax[k / 3] + kFixEmin - 1 - 1077);
   } else {
     R qi[5];
 #pragma unroll
@@ -3392,7 +3390,7 @@ struct Launch {
     }
     if (V.tsW) launchOrdered(kTsWeights<R>, shapeFor(V, V.nc), s, V);
   }
-  // The set-up of the fixed-point sums: the cells (View::fxScale; *slow is
+  // The set-up of the fixed-point sums: the cells (View::fxTop; *slow is
   // added the warps with a cell in FP64), then, with fxIdx and fxW, the weights.
   static void fixedSetup(const View<R> &V, int *slow, cudaStream_t s) {
     if constexpr (kFixedSums && !Layout<R>::packed) {

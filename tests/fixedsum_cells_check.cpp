@@ -1,4 +1,4 @@
-// A cell's least-squares sums in fixed point with the scales of its own weights
+// A cell's least-squares sums in fixed point with the scale of its own weights
 // (fixCellWeights), and as the FP64 loop forms them, over the cells read from
 // standard input: per line the member count, the own value, then (value, wx, wy,
 // wz) per member, as hexadecimal floats.  Prints "fp64" for a cell the fixed
@@ -24,20 +24,19 @@ int main() {
       if (std::scanf("%la %la %la %la", &q[k], &w[0][k], &w[1][k], &w[2][k]) != 4) return 1;
     int eq = fixOf(own).e;
     for (double x : q) eq = std::max(eq, fixOf(x).e);
-    const int packed = fixCellWeights(w[0].data(), w[1].data(), w[2].data(), n);
-    const bool fixed = packed != kFixNoWeights && eq != kFixBad;
+    const int top = fixCellWeights(w[0].data(), w[1].data(), w[2].data(), n);
+    const bool fixed = top != kFixNoWeights && eq != kFixBad;
     std::printf(fixed ? "fixed" : "fp64");
     if (fixed)
       for (int c = 0; c < 3; ++c) {
-        const int ew = fixWeightExp(packed, c);
         FixSum a{0, 0, 0};
         const FixNum o = fixOf(own);
         for (int k = 0; k < n; ++k) {
           const FixNum x = fixOf(q[k]);
-          const FixHalves d = fixSplit(fixAt(x.m, x.e, eq) - fixAt(o.m, o.e, eq)), h = fixSplit(fixWeight(w[c][k], ew));
+          const FixHalves d = fixSplit(fixAt(x.m, x.e, eq) - fixAt(o.m, o.e, eq)), h = fixSplit(fixWeight(w[c][k], top));
           fixAdd(a, h.hi, h.lo, h.hi + h.lo, d.hi, d.lo, d.hi + d.lo);
         }
-        std::printf(" %a", fixResult(a, fixScale(ew) - 55 + eq - 1077));
+        std::printf(" %a", fixResult(a, fixScale(top) - 55 + eq - 1077));
       }
     for (int c = 0; c < 3; ++c) {
       double s = 0.0;

@@ -8,7 +8,7 @@ from rocflu_gb300 import cases, gpu
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("precision,sides", [("mixed", (18, 19, 32, 33)), ("fp64", (12, 13, 21, 22)), ("fp64_exact", (12, 13))])
+@pytest.mark.parametrize("precision,sides", [("mixed", (16, 17, 32, 33)), ("fp64", (15, 16, 21, 22)), ("fp64_exact", (15, 16))])
 @pytest.mark.parametrize("reconst", [cases.RECONST_BJ, cases.RECONST_WENO_XYZ])
 def test_captured_and_host_launched_stages(gpu_lib, precision, sides, reconst):
     """Three steps replayed from the graph and three launched stage by stage:
