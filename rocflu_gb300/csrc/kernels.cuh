@@ -14,6 +14,7 @@
 #pragma once
 #include <algorithm>
 #include <climits>
+#include <mutex>
 #include <type_traits>
 #include <cuda_runtime.h>
 
@@ -3370,9 +3371,12 @@ struct Launch {
   }
   // The attribute belongs to the function, not to the context: it is only
   // raised, so that a context on a smaller mesh leaves a larger one's launches
-  // as they were.
+  // as they were.  Two host threads may create contexts at once: without the
+  // lock the smaller one's write could follow the larger one's.
   template <typename F>
   static void raiseSmem(F *f, size_t bytes) {
+    static std::mutex one;
+    std::lock_guard<std::mutex> lock(one);
     cudaFuncAttributes at;
     if (cudaFuncGetAttributes(&at, f) == cudaSuccess && (size_t)at.maxDynamicSharedSizeBytes >= bytes) return;
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
